@@ -20,7 +20,7 @@
 // fragment of the update is exactly the B fragment the next chunk's products need (bf16 copy in shared memory).
 // `gdn_chunk_finish_kernel` applies the gated RMSNorm * silu(z); `gdn_conv_tail_kernel` writes the conv history.
 // Chunks end at the block-aligned positions where a state snapshot is wanted (prefix cache), so snapshots are
-// plain copies of the running state.  All matrix products are bf16 x bf16 with fp32 accumulation.
+// plain copies of the running state.  Matrix products are bf16 x bf16 with fp32 accumulation (u: two terms per operand).
 #include <algorithm>
 
 #include "common.cuh"
@@ -79,12 +79,12 @@ TI_DEVICE float bf(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 // token and wait for them token by token); tiles stay row-major in shared memory and meet the tensor cores through
 // ldmatrix.trans (stores of transposed copies were 16-way bank conflicts); the diagonal blocks of the inverse are solved
 // in registers; beta and the decay are folded into the columns of the inverse, and the decays of q and k into the scan, so
-// that q and k fragments are written once per k-head.  4096 tokens, 16 k- and 48 v-heads of 128 x 128: 560 -> 190 us.
+// that q and k fragments are written once per k-head.  4096 tokens, 16 k- and 48 v-heads of 128 x 128: 560 -> 203 us.
 template <int DK, int DV>
 struct PrepSmem {
   static constexpr int QS = DK + 8, VS = DV + 8;   // bf16 row strides (16 bytes modulo 128: conflict-free ldmatrix)
   static constexpr int LS = kC + 8, TS = 36;       // fp32 row strides of the triangular matrix and of its half products
-  static constexpr size_t kBytes = (size_t)2 * kC * QS * 2 + (size_t)kC * VS * 2 + (size_t)kC * LS * 4 + 32 * TS * 4 +
+  static constexpr size_t kBytes = (size_t)2 * kC * QS * 2 + (size_t)2 * kC * VS * 2 + (size_t)kC * LS * 4 + 32 * TS * 4 +
                                    kMaxHpc * 3 * kC * 4;
 };
 
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(const __grid_
   extern __shared__ __align__(16) uint8_t smem[];
   __nv_bfloat16* qn = reinterpret_cast<__nv_bfloat16*>(smem);     // [64][QS]  q / |q| / sqrt(DK)
   __nv_bfloat16* kn = qn + kC * QS;                               // [64][QS]  k / |k|
-  __nv_bfloat16* vs = kn + kC * QS;                               // [64][VS]  v of one v-head
-  float* Lm = reinterpret_cast<float*>(vs + kC * VS);             // [64][LS]  L, then X
+  __nv_bfloat16* vs = kn + kC * QS;                               // [2][64][VS]  v of one v-head as two bf16 terms
+  float* Lm = reinterpret_cast<float*>(vs + 2 * kC * VS);         // [64][LS]  L, then X
   float* Tm = Lm + kC * LS;                                       // [32][TS]
   float* gates = Tm + 32 * TS;                                    // [hpc][3][64]: cumulative log decay, beta, beta exp(g)
 
@@ -295,6 +295,9 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(const __grid_
 #pragma unroll
           for (int e = 0; e < EV; ++e) y[e] = 0.f;
         store_packed<EV>(vs + (8 * warp + j) * VS + lane * EV, y);
+#pragma unroll
+        for (int e = 0; e < EV; ++e) y[e] -= round_bf16(y[e]);
+        store_packed<EV>(vs + kC * VS + (8 * warp + j) * VS + lane * EV, y);
       }
       if (h + 1 < hpc) load_v(vh + 1);               // requested ahead: a head's inverse hides the latency
     }
@@ -386,10 +389,12 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(const __grid_
     __syncthreads();
 
     // ---- E. u = (X b) v, -w = -(X b exp(g)) k: warp -> m-tile, half of the columns.  X is lower triangular: m-tile mt
-    //         meets mt + 1 k-tiles, so the two warps of a scheduler (warp & 3) take m-tiles i and 3 - i.
+    //         meets mt + 1 k-tiles, so the two warps of a scheduler (warp & 3) take m-tiles i and 3 - i.  u is kept in fp32
+    //         and is what the state is made of, so X b and v enter as two bf16 terms each (three products): against the
+    //         token-by-token rule in 64 bits outputs 0.40 -> 0.33 %, states 0.33 -> 0.23 %, for 18 us in 4096 tokens.
     {
       const int mt = warp < 4 ? warp : 7 - warp;
-      uint32_t xu[4][4], xw[4][4];
+      uint32_t xu[4][4], xl[4][4], xw[4][4];
 #pragma unroll
       for (int kt = 0; kt < 4; ++kt) {
         if (kt > mt) continue;
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(const __grid_
           const int col = 16 * kt + 2 * t + 8 * (i >> 1);
           const float2 x = *reinterpret_cast<const float2*>(Lm + (16 * mt + g + 8 * (i & 1)) * LS + col);
           const float2 b = *reinterpret_cast<const float2*>(bet + col), be = *reinterpret_cast<const float2*>(bge + col);
-          xu[kt][i] = pack_bf16(x.x * b.x, x.y * b.y);
+          split2(x.x * b.x, x.y * b.y, xu[kt][i], xl[kt][i]);
           xw[kt][i] = pack_bf16(-x.x * be.x, -x.y * be.y);
         }
       }
@@ -412,6 +417,11 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_kernel(const __grid_
           if (kt > mt) continue;
           uint32_t b[4];
           ldsm4t(b, vs + (16 * kt + (lane & 15)) * VS + 8 * nt + (lane >> 4) * 8);
+          mma_bf16_16816(acc[0], xu[kt][0], xu[kt][1], xu[kt][2], xu[kt][3], b[0], b[1]);
+          mma_bf16_16816(acc[1], xu[kt][0], xu[kt][1], xu[kt][2], xu[kt][3], b[2], b[3]);
+          mma_bf16_16816(acc[0], xl[kt][0], xl[kt][1], xl[kt][2], xl[kt][3], b[0], b[1]);
+          mma_bf16_16816(acc[1], xl[kt][0], xl[kt][1], xl[kt][2], xl[kt][3], b[2], b[3]);
+          ldsm4t(b, vs + kC * VS + (16 * kt + (lane & 15)) * VS + 8 * nt + (lane >> 4) * 8);
           mma_bf16_16816(acc[0], xu[kt][0], xu[kt][1], xu[kt][2], xu[kt][3], b[0], b[1]);
           mma_bf16_16816(acc[1], xu[kt][0], xu[kt][1], xu[kt][2], xu[kt][3], b[2], b[3]);
         }
