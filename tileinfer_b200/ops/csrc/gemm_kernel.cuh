@@ -1,5 +1,6 @@
-// W8A16 GEMM for prefill (many activation rows): y[M, N] = x[M, K] * W[N, K]^T on the 5th-generation tensor
-// cores (tcgen05.mma kind::i8, accumulators in tensor memory), fed by TMA.
+// W8A16 GEMM: y[M, N] = x[M, K] * W[N, K]^T on the 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators in tensor
+// memory), fed by TMA.  One output tile per CTA: batched decode, short products and experts; products of many tokens run on
+// pairs of CTAs (gemm_pair.cuh, which shares the operand layouts and epilogues).
 //
 // Replaces the reference's M > 1 path, which re-materialises a bf16 copy of the whole int8 weight on every
 // call and hands it to cuBLAS (kernels/splitk_gemv.py:243-247).
@@ -49,7 +50,7 @@ constexpr int kGemmProducerB = 6;
 #endif
 // bytes of operand ring per CTA.  96 lets two CTAs share an SM (TMEM: 2 x 256 columns), so that the epilogue of
 // one overlaps the main loop of the other.
-constexpr int kGemmShortRingKb = 96;       // the ring of products with a short k (see short_k)
+constexpr int kGemmShortRingKb = 96;       // the ring of routers' products and of bf16 experts
 // BN = tokens per CTA (TMEM columns per accumulator); BF16: bf16 weights and activations (one plane, one accumulator)
 // BMH = weight-row halves per CTA: 1 -> a 128-row tile; 2 -> a 256-row tile as two 128-row MMAs that share ONE
 // activation tile in shared memory (the bytes a CTA pulls through L2 per multiply-add drop by a third).
@@ -92,6 +93,7 @@ struct GemmParams {
   const int* num_tiles;
   int max_tiles, tiles_n, group_m; // token tiles; weight tiles per matrix; token tiles that share weight tiles in time
   int w_tiles;                     // 8-row weight tiles per matrix
+  int whole, cut, slices;          // gemm_pair.cuh: tiles with all of k, tiles cut along k, slices of a cut tile
 };
 
 // kind::i8 instruction descriptor: D = s32, A = int8 (K-major), B = int8 / uint8 (K-major), M = 128, N = BN
@@ -167,9 +169,31 @@ TI_DEVICE void gemm_epilogue4(const GemmParams& p, int m, int n, float4 v, uint2
       make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
 }
 
+// Residual of eight adjacent weight rows of one token, requested ahead of the epilogue: eight bf16 values (a) or eight fp32
+// ones (a, b).  Only where gemm_resid_vec says that the vectors are aligned, and for n + 8 <= N.
+struct ResidPre {
+  uint4 a, b;
+};
+TI_DEVICE bool gemm_resid_vec(const GemmParams& p) {
+  return p.epi == GEPI_RESID32 || (p.epi == GEPI_ROWPAR && (p.ldo & 7) == 0 && (p.N & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 &&
+                                   (reinterpret_cast<uintptr_t>(p.resid) & 15) == 0);
+}
+TI_DEVICE ResidPre gemm_resid_load(const GemmParams& p, int m, int n) {
+  ResidPre r = {};
+  if (p.epi == GEPI_RESID32) {
+    const uint4* src = reinterpret_cast<const uint4*>(p.ex.resid32 + (size_t)m * p.ldo + n);
+    r.a = src[0];
+    r.b = src[1];
+  } else {
+    r.a = *reinterpret_cast<const uint4*>(p.resid + (size_t)m * p.N + n);
+  }
+  return r;
+}
+
 // Eight adjacent weight rows n..n+7 (n a multiple of 8) of one token, straight from the accumulators: split-k
 // partial (fp32), or the fused epilogue.  Rows past N and rows that cannot be stored as one vector go one by one.
-TI_DEVICE void gemm_store8(const GemmParams& p, int m, int n, float4 a, float4 b, int S, int split) {
+// `pre`: the residual has been loaded (into `r0`).
+TI_DEVICE void gemm_store8(const GemmParams& p, int m, int n, float4 a, float4 b, int S, int split, bool pre = false, ResidPre r0 = ResidPre()) {
   if (S == 1 && p.ex.bias != nullptr) {            // N is a multiple of 8 here; with a split the reduction adds it
     const float4 c = __ldg(reinterpret_cast<const float4*>(p.ex.bias + n)), d = __ldg(reinterpret_cast<const float4*>(p.ex.bias + n + 4));
     a = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
@@ -214,7 +238,8 @@ TI_DEVICE void gemm_store8(const GemmParams& p, int m, int n, float4 a, float4 b
   }
   if (p.epi == GEPI_RESID32) {                     // N and ldo are multiples of 8 (checked by the launcher)
     const size_t at = (size_t)m * p.ldo + n;
-    const float4 ra = *reinterpret_cast<const float4*>(p.ex.resid32 + at), rb = *reinterpret_cast<const float4*>(p.ex.resid32 + at + 4);
+    if (!pre) r0 = gemm_resid_load(p, m, n);
+    const float4 ra = *reinterpret_cast<const float4*>(&r0.a), rb = *reinterpret_cast<const float4*>(&r0.b);
     float* dst = static_cast<float*>(p.out) + at;
     *reinterpret_cast<float4*>(dst) = make_float4(a.x + ra.x, a.y + ra.y, a.z + ra.z, a.w + ra.w);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(b.x + rb.x, b.y + rb.y, b.z + rb.z, b.w + rb.w);
@@ -240,7 +265,7 @@ TI_DEVICE void gemm_store8(const GemmParams& p, int m, int n, float4 a, float4 b
   if (p.epi == GEPI_ROWPAR) {
     const __nv_bfloat16* rs = p.resid + (size_t)m * p.N + n;
     if (vec) {
-      const uint4 q = *reinterpret_cast<const uint4*>(rs);
+      const uint4 q = pre ? r0.a : *reinterpret_cast<const uint4*>(rs);
       const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) { r[2 * i] += bf16lo(w4[i]); r[2 * i + 1] += bf16hi(w4[i]); }
@@ -554,38 +579,11 @@ static int launch_gemm(const GemmParams& p, dim3 grid, cudaStream_t st) {
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// bf16 products with many tokens and a short or medium k (at most 160 stages of 128 bytes) run two CTAs per SM with half
-// the ring each (TMEM: 2 x 256 columns), so that the epilogue of one overlaps the main loop of the other.  Measured at
-// 8192 tokens (us, one CTA -> two): k 512 213 -> 131, 2048 631 -> 516, 4096 2240 -> 2073, 10240 406 -> 348; 14336 and
-// more lose 6-10 %.
-static bool short_k(int KS, int BN, long long tiles) {
-  static const int limit = [] { const char* e = getenv("TI_GEMM_SHORT_K"); return e == nullptr ? 160 : atoi(e); }();
-  return BN == 128 && KS <= limit && tiles >= 2 * 148;
-}
-
-// 256-row tiles when the token tile is full-size and there are enough tiles to fill the GPU several times over
-// (TI_GEMM_BMH=1 / 2 forces a choice)
-static int pick_bmh(int M, int n_tiles) {
-  static const int forced = [] {
-    const char* e = getenv("TI_GEMM_BMH");
-    return e == nullptr ? 0 : atoi(e);
-  }();
-  if (forced == 1 || forced == 2) return n_tiles >= 32 ? forced : 1;
-  const long long tiles256 = (long long)((n_tiles * 8 + 255) / 256) * ((M + 127) / 128);
-  if (M <= 64) {
-    // few tokens: the limb planes are as many bytes per stage as the weights of a 128-row tile; with 256 rows they
-    // are half.  That pays only where no k split follows from halving the number of tiles.  Measured at 64 tokens on
-    // the 27B shapes (us, 128-row -> 256-row tiles): gate_up 43.6 -> 37.6 (136 tiles, no split), in_proj 23 -> 49
-    // (65 tiles in two k slices), down 47 -> 80, out_proj 36 -> 71.  TI_GEMM_BMH_SMALL=1 forces 256 rows.
-    static const int small = [] {
-      const char* e = getenv("TI_GEMM_BMH_SMALL");
-      return e == nullptr ? 0 : atoi(e);
-    }();
-    if (small && n_tiles >= 64) return 2;
-    return tiles256 >= 120 ? 2 : 1;          // enough 256-row tiles to fill the GPU without a k split (gate_up: 44 -> 38 us)
-  }
-  return (n_tiles >= 32 && tiles256 >= 2 * 148) ? 2 : 1;
-}
+// 256-row tiles for few tokens: the limb planes are as many bytes per stage as the weights of a 128-row tile; with 256 rows
+// they are half.  That pays only where no k split follows from halving the number of tiles.  Measured at 64 tokens on the 27B
+// shapes (us, 128-row -> 256-row tiles): gate_up 43.6 -> 37.6 (136 tiles, no split), in_proj 23 -> 49 (65 tiles in two k
+// slices), down 47 -> 80, out_proj 36 -> 71.
+static int pick_bmh(int M, int n_tiles) { return M <= 64 && (n_tiles * 8 + 255) / 256 * ((M + 127) / 128) >= 120 ? 2 : 1; }
 
 // k split that fills the 148 SMs when there are few output tiles; sets kb_per_split.  KB counts stages of 128 bytes
 // of k; a slice has at least 16 of them (TI_GEMM_SPLIT_STAGES).  Measured at 64 tokens on N = 5120 (us): K = 6144

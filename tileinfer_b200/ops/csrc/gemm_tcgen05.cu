@@ -1,5 +1,5 @@
 // Entry points of the tcgen05 products (gemm_kernel.cuh) and the activation quantisation of the int8 form.
-#include "gemm_kernel.cuh"
+#include "gemm_pair.cuh"
 
 namespace ti {
 
@@ -170,7 +170,8 @@ int ti_quant_rows(const void* x, int ldx, const void* norm_w, float eps, int M, 
 
 // y = x W^T for tiled int8 weights `w` ([n_tiles][K/64][8][64]) and the limb planes of x.
 // `part` / `tile_count`: split-k workspace (fp32 [S][M][N]) and zeroed per-tile counters, may be null (no split);
-// `part_bytes` / `n_count` are their capacities.  The token tile (32 / 64 / 128) and the k split follow from M, N.
+// `part_bytes` / `n_count` are their capacities.  The kernel (gemm_pair.cuh for many tokens, gemm_kernel.cuh), the token tile and the
+// k split follow from M, N, K.
 int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, const void* xh, const void* xl,
                   const void* xscale, int M, const void* resid, void* out, int ldo, int epi, void* status, void* part,
                   size_t part_bytes, void* tile_count, int n_count, const ti::GemmEpilogue* ex, void* stream) {
@@ -179,12 +180,15 @@ int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, 
   ti::GemmParams p = {};
   const int KB = K / 64, KS = (KB + ti::kKS - 1) / ti::kKS;      // 64-byte slabs of the weight layout; 128-byte stages
   const int BN = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
-  const int BMH = ti::pick_bmh(M, n_tiles);
+  const bool may_cut = ti::pair_may_cut(part, part_bytes, tile_count, n_count);
+  const ti::PairPlan plan = ti::pair_plan(M, n_tiles, KS, 128, may_cut);
+  const bool pair = ti::pair_serves(M, N, KS);
+  const int BMH = pair ? 1 : ti::pick_bmh(M, n_tiles);
   int rc = ti::cached_map(&p.map_w, w, KB, n_tiles, BMH == 2 ? -32 : 0);
   if (rc) return rc;
-  rc = ti::cached_map(&p.map_xh, xh, K, M, BN);
+  rc = ti::cached_map(&p.map_xh, xh, K, M, pair ? 64 : BN);
   if (rc) return rc;
-  rc = ti::cached_map(&p.map_xl, xl, K, M, BN);
+  rc = ti::cached_map(&p.map_xl, xl, K, M, pair ? 64 : BN);
   if (rc) return rc;
   p.xscale = (const float*)xscale;
   p.wscale = (const __nv_bfloat16*)wscale;
@@ -198,14 +202,17 @@ int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, 
   p.epi = epi;
   rc = ti::set_epilogue(p, ex);
   if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (pair) {
+    ti::pair_apply(p, plan, n_tiles, 128, part, tile_count);
+    return ti::launch_pair<128, false>(p, st);
+  }
   const int rows = ti::kBM * BMH;
   const int tiles_n = (n_tiles * 8 + rows - 1) / rows, tiles_m = (M + BN - 1) / BN;
   const int S = ti::plan_split(p, KS, tiles_n * tiles_m, M, N, ldo, part, part_bytes, tile_count, n_count);
   dim3 grid(tiles_m, tiles_n, S);
-  cudaStream_t st = (cudaStream_t)stream;
   if (BMH == 2 && BN == 32) return ti::launch_gemm<32, false, 2>(p, grid, st);
   if (BMH == 2 && BN == 64) return ti::launch_gemm<64, false, 2>(p, grid, st);
-  if (BMH == 2) return ti::launch_gemm<128, false, 2>(p, grid, st);
   if (BN == 32) return ti::launch_gemm<32, false>(p, grid, st);
   if (BN == 64) return ti::launch_gemm<64, false>(p, grid, st);
   return ti::launch_gemm<128, false>(p, grid, st);
@@ -222,10 +229,14 @@ int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M,
   const int KB = K / 32, KS = (KB + ti::kKS - 1) / ti::kKS;    // 64-byte slabs; 128-byte stages
   // a single weight tile (a router): smaller token tiles, so that there are enough of them for all SMs
   const int BN = M <= 32 || (N <= 128 && M <= 64 * 148) ? 32 : (M <= 64 || N <= 128 ? 64 : 128);
-  const int BMH = ti::pick_bmh(M, n_tiles);
+  const bool may_cut = ti::pair_may_cut(part, part_bytes, tile_count, n_count);
+  const int NT = ti::pair_tokens_bf16(M, n_tiles, KS, may_cut);
+  const ti::PairPlan plan = ti::pair_plan(M, n_tiles, KS, NT, may_cut);
+  const bool pair = ti::pair_serves(M, N, KS);
+  const int BMH = pair ? 1 : ti::pick_bmh(M, n_tiles);
   int rc = ti::cached_map(&p.map_w, w, KB, n_tiles, BMH == 2 ? -32 : 0);
   if (rc) return rc;
-  rc = ti::cached_map(&p.map_xh, x, 2 * K, M, BN);
+  rc = ti::cached_map(&p.map_xh, x, 2 * K, M, pair ? NT / 2 : BN);
   if (rc) return rc;
   p.resid = (const __nv_bfloat16*)resid;
   p.out = out;
@@ -237,17 +248,18 @@ int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M,
   p.epi = epi;
   rc = ti::set_epilogue(p, ex);
   if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (pair) {
+    ti::pair_apply(p, plan, n_tiles, NT, part, tile_count);
+    return NT == 256 ? ti::launch_pair<256, true>(p, st) : ti::launch_pair<128, true>(p, st);
+  }
   const int rows = ti::kBM * BMH;
   const int tiles_n = (n_tiles * 8 + rows - 1) / rows, tiles_m = (M + BN - 1) / BN;
   const int S = ti::plan_split(p, KS, tiles_n * tiles_m, M, N, ldo, part, part_bytes, tile_count, n_count);
   dim3 grid(tiles_m, tiles_n, S);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (S == 1 && ti::short_k(KS, BN, (long long)tiles_n * tiles_m))
-    return BMH == 2 ? ti::launch_gemm<128, true, 2, ti::kGemmShortRingKb>(p, grid, st) : ti::launch_gemm<128, true, 1, ti::kGemmShortRingKb>(p, grid, st);
   if (N <= 128 && M > 64 && BN == 32) return ti::launch_gemm<32, true, 1, ti::kGemmShortRingKb>(p, grid, st);   // two CTAs per SM
   if (BMH == 2 && BN == 32) return ti::launch_gemm<32, true, 2>(p, grid, st);
   if (BMH == 2 && BN == 64) return ti::launch_gemm<64, true, 2>(p, grid, st);
-  if (BMH == 2) return ti::launch_gemm<128, true, 2>(p, grid, st);
   if (BN == 32) return ti::launch_gemm<32, true>(p, grid, st);
   if (BN == 64) return ti::launch_gemm<64, true>(p, grid, st);
   return ti::launch_gemm<128, true>(p, grid, st);
