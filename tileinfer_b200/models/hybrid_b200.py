@@ -471,6 +471,12 @@ class _StepMixin:
                     cp.wf, cp.qf, cp.mf, cp.kf, cp.u, cp.gamma = (ptr(b) for b in ws)
                     F.gdn_chunked(cp, S, T, self.dk, self.dv, self.state_bf16)
                     self._launches += 4
+                    if x.one is not None:
+                        # one-token sequences; after the chunk kernels, which leave these rows of the output undefined
+                        p.slots, p.toks = ptr(x.one[0]), ptr(x.one[1])
+                        p.snap_rel, p.snap_idx, p.num_snap = None, None, 0
+                        F.gdn_step(p, x.one.shape[1], self.dk, self.dv, self.state_bf16, single=True)
+                        self._launches += 1
                 else:
                     F.gdn_step(p, S, self.dk, self.dv, self.state_bf16, split=self.gdn_split and T > S, single=T == S)
                     self._launches += 1
@@ -563,8 +569,14 @@ class _RunMixin(DeviceRuntime):
             rel_l = ent_l = None
             if snaps:
                 rel_l, ent_l = rel.tolist(), idx.tolist()
-            ck, seq_ck = F.gdn_chunk_table(batch.cu_seqlens, rel_l, ent_l)
+            # running sequences beside a prompt take the decode kernels: as chunks of one token each would cost as much as
+            # 64 tokens (29 of them beside 1031 prompt tokens: 350 of 600 us per layer)
+            one = [s for s, n in enumerate(lens) if n == 1 and not (batch.snapshot_at and batch.snapshot_at[s])]
+            ck, seq_ck = F.gdn_chunk_table(batch.cu_seqlens, rel_l, ent_l, skip=one)
             x.ck, x.seq_ck = ck.to(dev, non_blocking=True), seq_ck.to(dev, non_blocking=True)
+            if one:
+                x.one = torch.tensor([[batch.state_slots[s] for s in one], [batch.cu_seqlens[s] for s in one]],
+                                     dtype=torch.int32).to(dev, non_blocking=True)
 
     def _finish_step(self, x: StepCtx):
         # snapshots stay on the device (a 27B snapshot is 151 MB; 64 of them are 5 % of a B200's memory)

@@ -26,6 +26,7 @@ class StepCtx:
     tiles = None            # [3, n] query tiles of the tcgen05 prefill attention (sequence, first token, tokens)
     ck = None               # [4, nc] chunk table of the chunked DeltaNet prefill (None: token-serial kernel)
     seq_ck = None
+    one = None              # [2, n] state slot and flat token of the one-token sequences beside chunked ones
 
 
 class DeviceRuntime:

@@ -41,7 +41,12 @@ struct GdnParams {
   float eps;
   const int* snap_idx;         // [S, NS] index of the snapshot buffer entry of (sequence, point), or nullptr (s * NS + j)
   unsigned* status;            // error bits (a bounded wait that ran out); may be nullptr
+  const int* toks;             // nullptr, or [S]: sequence s has the one token toks[s] (`cu` is not read; single-pass kernels)
 };
+
+// flat token range of sequence s
+TI_DEVICE int first_token(const GdnParams& p, int s) { return p.toks ? p.toks[s] : (p.cu ? p.cu[s] : s); }
+TI_DEVICE int end_token(const GdnParams& p, int s) { return p.toks ? p.toks[s] + 1 : (p.cu ? p.cu[s + 1] : s + 1); }
 
 TI_DEVICE size_t snap_entry(const GdnParams& p, int s, int j) {
   return p.snap_idx != nullptr ? (size_t)p.snap_idx[s * p.num_snap + j] : (size_t)s * p.num_snap + j;
@@ -117,7 +122,7 @@ __global__ void __launch_bounds__(DV * 4) gdn_token_kernel(const __grid_constant
   struct Inputs { float x0, x1, x2, x3, a, b, z; };
   auto fetch = [&](int seq) {
     Inputs in{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int tokn = p.cu ? p.cu[seq] : seq;
+    const int tokn = first_token(p, seq);
     const __nv_bfloat16* rown = p.proj + (size_t)tokn * p.ld;
     const __nv_bfloat16* csn = p.conv_state + ((size_t)p.slots[seq] * p.hv + vh) * 3 * NCH;
     if (tid < NCH) {
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(DV * 4) gdn_token_kernel(const __grid_constant
   for (int s = blockIdx.y; s < num_seqs; s += gridDim.y, ++k) {
     // cu / slots are written by host copies that precede every kernel of the step; the recurrent state
     // and conv history were last written one step ago: all of this may be read before pdl_wait()
-    const int t0 = p.cu ? p.cu[s] : s, t1 = p.cu ? p.cu[s + 1] : s + 1;
+    const int t0 = first_token(p, s), t1 = end_token(p, s);
     const int slot = p.slots[s];
     ST* Sp = static_cast<ST*>(p.state) + ((size_t)slot * p.hv + vh) * DK * DV;
     ST* sb = sbuf0 + (size_t)(k & 1) * DK * DV;
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(128, sizeof(ST) == 4 ? 8 : 6) gdn_token_split_
   const int part = blockIdx.x % NSPL, vh = blockIdx.x / NSPL, s = blockIdx.y;
   const int kh = vh / (p.hv / p.hk);
   const int slot = p.slots[s];
-  const int tok = p.cu ? p.cu[s] : s;
+  const int tok = first_token(p, s);
   ST* Sp = static_cast<ST*>(p.state) + ((size_t)slot * p.hv + vh) * DK * DV + part * CB + c;
   float S[DPT];
 #pragma unroll
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(256) gdn_finish_kernel(const __grid_constant__
   pdl_wait();
   if (item >= num_seqs * p.hv) return;
   const int s = item / p.hv, vh = item - s * p.hv;
-  const int tok = p.cu ? p.cu[s] : s;
+  const int tok = first_token(p, s);
   __nv_bfloat16* o = p.out + (size_t)tok * p.hv * DV + vh * DV + lane * E;
   const __nv_bfloat16* z = p.proj + (size_t)tok * p.ld + 2 * p.hk * DK + p.hv * DV + vh * DV + lane * E;
   float v[E], ss = 0.f;
@@ -735,7 +740,7 @@ int ti_gdn_params_size() { return (int)sizeof(ti::GdnParams); }
 // several sequences when snapshots are wanted, or with split 3).
 int ti_gdn_step(const ti::GdnParams* p, int num_seqs, int dk, int dv, int state_bf16, int split, void* stream) {
   if (num_seqs <= 0) return 0;
-  if (p->hv % p->hk) return -2;
+  if (p->hv % p->hk || (p->toks != nullptr && split < 2)) return -2;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e;
   if (split >= 2) {                     // one token per sequence: the single-pass decode kernel

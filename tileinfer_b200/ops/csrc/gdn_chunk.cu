@@ -52,7 +52,8 @@ struct GdnChunkParams {
   const int* ck_tok0;          // [nc] first flat token
   const int* ck_ntok;          // [nc] 1..64
   const int* ck_snap;          // [nc] snapshot entry to write after this chunk, or -1
-  const int* seq_ck;           // [S+1] chunk range of every sequence
+  const int* seq_ck;           // [S+1] chunk range of every sequence; one without chunks is left alone (a one-token sequence
+                               // of a mixed step, which the decode kernels of gdn.cu advance)
   // workspace, fragment order (index ch = chunk * hv + v-head, ck = chunk * hk + k-head)
   uint4* wf;                   // [ch][4 m-tiles][DK/16 k-tiles][32 lanes]   A fragments of -w  (64 x DK)
   uint4* qf;                   // [ck][4][DK/16][32]                         A fragments of q DK^-1/2
@@ -475,6 +476,8 @@ __global__ void __launch_bounds__(128, 2) gdn_chunk_scan_kernel(const __grid_con
 
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int vh = blockIdx.x / NB, dv0 = (blockIdx.x % NB) * DVB, s = blockIdx.y, kh = vh / (p.hv / p.hk);
+  const int c_lo = p.seq_ck[s], c_hi = p.seq_ck[s + 1];
+  if (c_lo == c_hi) return;                                      // not this kernel's sequence: its state is not touched
   const int slot = p.slots[s];
   ST* Sp = static_cast<ST*>(p.state) + ((size_t)slot * p.hv + vh) * DK * DV;
   const int dk0 = w * (DK / 4);                                  // this warp's slice of dk in the state update
@@ -531,8 +534,7 @@ __global__ void __launch_bounds__(128, 2) gdn_chunk_scan_kernel(const __grid_con
     ek0 = __ldg(sc + 4 + kC + 16 * w + g);
     ek1 = __ldg(sc + 4 + kC + 16 * w + g + 8);
   };
-  const int c_lo = p.seq_ck[s], c_hi = p.seq_ck[s + 1];
-  if (c_lo < c_hi) load_a(c_lo);
+  load_a(c_lo);
   __syncthreads();
 
   for (int ci = c_lo; ci < c_hi; ++ci) {
@@ -701,6 +703,7 @@ __global__ void __launch_bounds__(128) gdn_conv_tail_kernel(const __grid_constan
   const int s = blockIdx.x, vh = blockIdx.y, z = blockIdx.z;
   const int NCH = 2 * DK + DV;
   const int kh = vh / (p.hv / p.hk);
+  if (p.seq_ck[s] == p.seq_ck[s + 1]) return;
   const int t0 = p.cu[s], t1 = p.cu[s + 1];
   int n = t1 - t0;
   __nv_bfloat16* hist = p.conv_state + ((size_t)p.slots[s] * p.hv + vh) * 3 * NCH;
@@ -767,7 +770,8 @@ int ti_gdn_chunk_ws_bytes(int dk, int dv, int which) {
 }
 
 // Chunked prefill of the gated DeltaNet mixer for a flattened batch (see the file comment): prepare, scan, finish,
-// conv tail.  `num_seqs` sequences, `T` tokens; the chunk table in `p` must cover every token exactly once.
+// conv tail.  `num_seqs` sequences, `T` tokens; the chunk table in `p` covers every token of a sequence, or none (its rows of
+// `out` are then undefined).
 int ti_gdn_chunked(const ti::GdnChunkParams* p, int num_seqs, int T, int dk, int dv, int state_bf16, void* stream) {
   if (num_seqs <= 0 || p->nc <= 0) return 0;
   if (p->hv % p->hk) return -2;

@@ -43,7 +43,8 @@ GEMV_UNITS_PER_WARP = int(os.environ.get("TI_GEMV_UPW", "4"))
 class GdnParams(ctypes.Structure):
     _fields_ = [("proj", _P), ("conv_w", _P), ("neg_a_exp", _P), ("dt_bias", _P), ("norm_w", _P), ("state", _P),
                 ("conv_state", _P), ("slots", _P), ("cu", _P), ("out", _P), ("snap_rel", _P), ("snap_state", _P),
-                ("snap_conv", _P), ("ld", _I), ("hk", _I), ("hv", _I), ("num_snap", _I), ("eps", _F), ("snap_idx", _P), ("status", _P)]
+                ("snap_conv", _P), ("ld", _I), ("hk", _I), ("hv", _I), ("num_snap", _I), ("eps", _F), ("snap_idx", _P), ("status", _P),
+                ("toks", _P)]
 
 
 class GdnChunkParams(ctypes.Structure):
@@ -593,13 +594,18 @@ def gdn_step(p: GdnParams, num_seqs: int, dk: int, dv: int, state_bf16: bool, sp
 GDN_CHUNK = 64
 
 
-def gdn_chunk_table(cu_seqlens, snapshot_rel=None, snapshot_entry=None):
+def gdn_chunk_table(cu_seqlens, snapshot_rel=None, snapshot_entry=None, skip=()):
     """Chunk table of the chunked DeltaNet prefill: every sequence is cut into chunks of at most 64 tokens that
     also end wherever a state snapshot is wanted.  `snapshot_rel[s]`: token counts (relative to the start of the
-    step) after which sequence s snapshots, `snapshot_entry[s]`: the entries of the snapshot buffers.
+    step) after which sequence s snapshots, `snapshot_entry[s]`: the entries of the snapshot buffers.  Sequences in `skip`
+    get no chunks.
     Returns int32 tensors (ck [4, nc] = sequence | first flat token | tokens | snapshot entry or -1, seq_ck [S+1])."""
     seq, tok0, ntok, snap, seq_ck = [], [], [], [], [0]
+    skip = set(skip)
     for s in range(len(cu_seqlens) - 1):
+        if s in skip:
+            seq_ck.append(len(seq))
+            continue
         t0, t1 = cu_seqlens[s], cu_seqlens[s + 1]
         pts = {}
         if snapshot_rel is not None:
