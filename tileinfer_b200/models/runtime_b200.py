@@ -8,7 +8,9 @@ Device half of the reference's ModelRunner (engine/model_runner.py:135-498).
 from __future__ import annotations
 
 import gc
+import struct
 
+import numpy as np
 import torch
 
 from ..ops import functional as F
@@ -27,6 +29,23 @@ class StepCtx:
     ck = None               # [4, nc] chunk table of the chunked DeltaNet prefill (None: token-serial kernel)
     seq_ck = None
     one = None              # [2, n] state slot and flat token of the one-token sequences beside chunked ones
+
+
+def _words(shape, size: int) -> int:
+    n = size // 4
+    for d in shape:
+        n *= d
+    return n
+
+
+def _layout(parts):
+    """{name: (first 32-bit word, shape, bytes per value)} of parts packed one after the other, each on a 256-byte boundary as
+    an allocation of its own would be, and the words in all."""
+    at, out = 0, {}
+    for name, shape, size in parts:
+        out[name] = (at, shape, size)
+        at += -(-_words(shape, size) // 64) * 64
+    return out, at
 
 
 class DeviceRuntime:
@@ -105,16 +124,46 @@ class DeviceRuntime:
         return False
 
     def _alloc_inputs(self, T: int, S: int, max_blocks: int, num_qg: int, nsplit: int) -> StepCtx:
-        """The inputs every model's step has: tokens, positions, cache slots, block tables, query groups."""
-        dev, x = self.dev, StepCtx()
+        """The inputs every model's step has: tokens, positions, cache slots, block tables, query groups (seq, tok0, ntok).
+        They are parts of one buffer, so that one host -> device copy brings a step's inputs (`_host_inputs`)."""
+        x = StepCtx()
         x.T, x.S, x.max_blocks, x.num_qg, x.nsplit = T, S, max_blocks, num_qg, nsplit
-        x.ids = torch.zeros(T, dtype=torch.long, device=dev)
-        x.positions = torch.zeros(T, dtype=torch.int32, device=dev)
-        x.slot_mapping = torch.full((T,), -1, dtype=torch.long, device=dev)
-        x.slots = torch.zeros(S, dtype=torch.int32, device=dev)
-        x.block_tables = torch.zeros(S, max_blocks, dtype=torch.int32, device=dev)
-        x.qg = torch.zeros(3, max(num_qg, 1), dtype=torch.int32, device=dev)      # seq, tok0, ntok
+        x.layout, words = _layout((("ids", (T,), 8), ("slot_mapping", (T,), 8), ("positions", (T,), 4), ("slots", (S,), 4),
+                                   ("qg", (3, max(num_qg, 1)), 4), ("block_tables", (S, max_blocks), 4)))
+        x.inputs = torch.empty(words, dtype=torch.int32, device=self.dev)
+        for name, (at, shape, size) in x.layout.items():
+            t = x.inputs[at:at + _words(shape, size)]
+            setattr(x, name, (t.view(torch.long) if size == 8 else t).view(shape))
         return x
+
+    @staticmethod
+    def _host_inputs(x: StepCtx, buf: np.ndarray) -> dict:
+        """numpy views of the parts of the host buffer `buf`, laid out like x.inputs."""
+        return {name: buf[at:at + _words(shape, size)].view(np.int64 if size == 8 else np.int32).reshape(shape)
+                for name, (at, shape, size) in x.layout.items()}
+
+    @staticmethod
+    def _fill_batch(h: dict, batch):
+        """The batch's tokens, positions, slots and block tables into the views of `_host_inputs`."""
+        n, S = batch.cu_seqlens[-1], batch.num_seqs
+        h["ids"][:n] = batch.input_ids.cpu().numpy()
+        h["positions"][:n] = batch.positions.cpu().numpy()
+        h["slot_mapping"][:n] = batch.slot_mapping.cpu().numpy()
+        h["slots"][:S] = batch.state_slots
+        tables = h["block_tables"]
+        pitch = tables.strides[0]
+        for s, b in enumerate(batch.block_tables):           # (a tensor per row took 12 us, this takes 1)
+            struct.pack_into(f"{len(b)}i", tables, s * pitch, *b)
+
+    def _upload(self, *arrays) -> list:
+        """Device copies of some small int32 arrays (anything numpy takes; None stays None): one transfer for all of them."""
+        arrays = [None if a is None else np.asarray(a, dtype=np.int32) for a in arrays]
+        layout, words = _layout([(i, a.shape, 4) for i, a in enumerate(arrays) if a is not None])
+        buf = np.empty(words, dtype=np.int32)
+        for i, (at, shape, _) in layout.items():
+            buf[at:at + arrays[i].size] = arrays[i].reshape(-1)
+        dev = torch.from_numpy(buf).to(self.dev, non_blocking=True)
+        return [None if a is None else dev[layout[i][0]:layout[i][0] + a.size].view(a.shape) for i, a in enumerate(arrays)]
 
     def _topk_rows(self, logits, n, k):
         """Per-rank top-k (+ fused candidate exchange); rows in chunks of the peer buffer capacity."""
@@ -155,31 +204,23 @@ class DeviceRuntime:
         """Eager step over a flattened batch (prefill chunks and/or decode tokens).  Returns the
         residual-stream rows of the last token of every sequence (or of `batch.out_rows`); the final
         norm belongs to the vocabulary product."""
-        dev = self.dev
         S, T = batch.num_seqs, batch.cu_seqlens[-1]
         qg_seq, qg_tok0, qg_ntok, tiles = self._fill_ctx(None, batch)
         nq = len(qg_seq)
         max_blocks = max(len(b) for b in batch.block_tables)
         nsplit = 1 if nq * self.hkv >= F.NUM_SMS else max(1, min(32, -(-8 * F.NUM_SMS // (max(nq, 1) * self.hkv))))
         x = self._alloc_ctx(T, S, max_blocks, nq, nsplit)
-        x.ids.copy_(batch.input_ids, non_blocking=True)
-        x.positions.copy_(batch.positions.to(torch.int32), non_blocking=True)
-        x.slot_mapping.copy_(batch.slot_mapping, non_blocking=True)
-        x.slots.copy_(torch.tensor(batch.state_slots, dtype=torch.int32), non_blocking=True)
-        x.cu = torch.tensor(batch.cu_seqlens, dtype=torch.int32, device=dev)
-        bt = torch.zeros(S, max_blocks, dtype=torch.int32)
-        for s, b in enumerate(batch.block_tables):
-            bt[s, :len(b)] = torch.tensor(b, dtype=torch.int32)
-        x.block_tables.copy_(bt, non_blocking=True)
+        buf = np.zeros(x.inputs.numel(), dtype=np.int32)
+        h = self._host_inputs(x, buf)
+        self._fill_batch(h, batch)
         if nq:
-            x.qg.copy_(torch.tensor([qg_seq, qg_tok0, qg_ntok], dtype=torch.int32), non_blocking=True)
-        if tiles:
-            x.tiles = torch.tensor([[t[1] for t in tiles], [t[2] for t in tiles], [t[3] for t in tiles]],
-                                   dtype=torch.int32).to(dev, non_blocking=True)
+            h["qg"][:] = (qg_seq, qg_tok0, qg_ntok)
+        x.inputs.copy_(torch.from_numpy(buf), non_blocking=True)
+        rows = batch.out_rows if batch.out_rows is not None else [c - 1 for c in batch.cu_seqlens[1:]]
+        x.cu, x.tiles, rows = self._upload(batch.cu_seqlens, [[t[i] for t in tiles] for i in (1, 2, 3)] if tiles else None, rows)
         self._prepare_step(x, batch)
         cur = self._run_layers(x)
-        rows = batch.out_rows if batch.out_rows is not None else [c - 1 for c in batch.cu_seqlens[1:]]
-        hidden = cur[torch.tensor(rows, dtype=torch.long, device=dev)]
+        hidden = cur.index_select(0, rows)
         self._finish_step(x)
         self.host_steps += 1
         return hidden
@@ -234,19 +275,16 @@ class DeviceRuntime:
         base = next((v for kk, v in self.graphs.items() if kk[0] == B), None)
         g = StepCtx()
         if base is not None:      # same bucket, other k: share the input tensors
-            g.x = base.x
-            g.host = base.host
+            g.x, g.host, g.views, g.uploaded = base.x, base.host, base.views, base.uploaded
         else:
             g.x = self._alloc_ctx(B, B, self.graph_max_blocks, B, nsplit)
             x = g.x
-            g.host = {
-                "ids": torch.zeros(B, dtype=torch.long).pin_memory(),
-                "positions": torch.zeros(B, dtype=torch.int32).pin_memory(),
-                "slot_mapping": torch.full((B,), -1, dtype=torch.long).pin_memory(),
-                "slots": torch.full((B,), self.padding_slot, dtype=torch.int32).pin_memory(),
-                "block_tables": torch.zeros(B, self.graph_max_blocks, dtype=torch.int32).pin_memory(),
-                "qg": torch.zeros(3, B, dtype=torch.int32).pin_memory(),
-            }
+            g.host = {"inputs": torch.zeros(x.inputs.numel(), dtype=torch.int32).pin_memory()}
+            g.views = self._host_inputs(x, g.host["inputs"].numpy())
+            g.views["qg"][:2] = np.arange(B)
+            g.uploaded = torch.cuda.Event()
+            x.inputs.zero_()
+            x.slot_mapping.fill_(-1)
             x.slots.fill_(self.padding_slot)
         x = g.x
         g.logits = None if fa else torch.zeros(B, self.v_local, dtype=torch.float32, device=dev)
@@ -318,10 +356,11 @@ class DeviceRuntime:
         """Parameter blocks of the edit and sample kernels for `n` rows whose candidates `topk_state` produces."""
         dev, e = self.dev, self._edit_buffers()
         t = StepCtx()
-        t.fpar = torch.zeros(3, n, dtype=torch.float32, device=dev)            # temperature | top_p | u
-        t.ipar = torch.full((2, n), -1, dtype=torch.int32, device=dev)         # top_k | edit slot
-        t.h_fpar = torch.zeros(3, n, dtype=torch.float32).pin_memory()
-        t.h_ipar = torch.full((2, n), -1, dtype=torch.int32).pin_memory()
+        t.par = torch.zeros(5, n, dtype=torch.int32, device=dev)
+        t.h_par = torch.zeros(5, n, dtype=torch.int32).pin_memory()
+        t.fpar, t.h_fpar = t.par[:3].view(torch.float32), t.h_par[:3].view(torch.float32)      # temperature | top_p | u
+        t.ipar, t.h_ipar = t.par[3:].fill_(-1), t.h_par[3:].fill_(-1)                          # top_k | edit slot
+        t.np_f, t.np_i = t.h_fpar.numpy(), t.h_ipar.numpy()
         t.tok = torch.zeros(n + 1, dtype=torch.int32, device=dev)
         t.h_tok = torch.zeros(n + 1, dtype=torch.int32).pin_memory()
         ep = EditParams()
@@ -339,13 +378,10 @@ class DeviceRuntime:
 
     def _upload_sampling(self, t, n, spec):
         """Host -> device copies of a step's sampling parameters and logit edits (pinned staging, asynchronous)."""
-        hf, hi = t.h_fpar, t.h_ipar
-        hf[0].zero_()                                   # padding rows: greedy
-        hi[1].fill_(-1)
-        hf[0, :n] = torch.tensor(spec["temperature"], dtype=torch.float32)
-        hf[1, :n] = torch.tensor(spec["top_p"], dtype=torch.float32)
-        hf[2, :n] = torch.tensor(spec["u"], dtype=torch.float32)
-        hi[0, :n] = torch.tensor(spec["top_k"], dtype=torch.int32)
+        hf, hi = t.np_f, t.np_i
+        hf[0, n:] = 0                                   # padding rows: greedy
+        hi[1] = -1
+        hf[0, :n], hf[1, :n], hf[2, :n], hi[0, :n] = spec["temperature"], spec["top_p"], spec["u"], spec["top_k"]
         edits = spec.get("edits") or []
         if edits:
             e = self._edit_buffers()
@@ -363,8 +399,7 @@ class DeviceRuntime:
                     e.h_pen[slot, :cnt] = pen[:cnt]
                     e.pen_ids[slot, :cnt].copy_(e.h_pen[slot, :cnt], non_blocking=True)
             e.meta.copy_(e.h_meta, non_blocking=True)
-        t.fpar.copy_(hf, non_blocking=True)
-        t.ipar.copy_(hi, non_blocking=True)
+        t.par.copy_(t.h_par, non_blocking=True)
 
     def _read_tokens(self, t, n) -> list:
         """The step's only device -> host copy: n token ids and the communicator's status word."""
@@ -377,27 +412,15 @@ class DeviceRuntime:
         n = batch.num_seqs
         g = self.decode_graph(n, k, edits=keep_logits or bool(spec and spec.get("edits")))
         self._last_graph = g
-        h, x = g.host, g.x
-        h["ids"][:n] = batch.input_ids
-        h["positions"][:n] = batch.positions
-        h["slot_mapping"][:n] = batch.slot_mapping
+        h, x = g.views, g.x
+        g.uploaded.synchronize()                     # an earlier step's copy may still be reading the staging buffer
+        self._fill_batch(h, batch)
         h["slot_mapping"][n:] = -1
-        h["slots"][:n] = torch.tensor(batch.state_slots, dtype=torch.int32)
         h["slots"][n:] = self.padding_slot
-        bt = h["block_tables"]
-        for s, b in enumerate(batch.block_tables):
-            bt[s, :len(b)] = torch.tensor(b, dtype=torch.int32)
-        qg = h["qg"]
-        qg[0, :n] = torch.arange(n, dtype=torch.int32)
-        qg[1, :n] = torch.arange(n, dtype=torch.int32)
-        qg[2, :n] = 1
-        qg[2, n:] = 0
-        x.ids.copy_(h["ids"], non_blocking=True)
-        x.positions.copy_(h["positions"], non_blocking=True)
-        x.slot_mapping.copy_(h["slot_mapping"], non_blocking=True)
-        x.slots.copy_(h["slots"], non_blocking=True)
-        x.block_tables.copy_(bt, non_blocking=True)
-        x.qg.copy_(qg, non_blocking=True)
+        h["qg"][2, :n], h["qg"][2, n:] = 1, 0
+        end = x.layout["block_tables"][0] + n * x.max_blocks         # the tables are the last part: those of n sequences
+        x.inputs[:end].copy_(g.host["inputs"][:end], non_blocking=True)
+        g.uploaded.record()
         if spec is not None:
             self._upload_sampling(g.samp, n, spec)
         if self.peer is not None:
@@ -418,7 +441,8 @@ class DeviceRuntime:
         rows = batch.out_rows if batch.out_rows is not None else [e - 1 for e in batch.cu_seqlens[1:]]
         if self._graph_serves(batch):
             self._decode_graph_step(batch, 1, keep_logits=True)
-            return self._last_graph.logits[rows]
+            logits = self._last_graph.logits
+            return logits[:len(rows)].clone() if rows == list(range(len(rows))) else logits[rows]
         hidden = self.forward(batch)
         return self.logits(hidden) if rows else torch.empty(0, self.v_local, device=self.dev)
 
@@ -458,8 +482,9 @@ class DeviceRuntime:
                 return self._read_tokens(self._last_graph.samp, n)
         else:
             hidden = self.forward(batch)
-            rows = torch.tensor(sample_rows, dtype=torch.long, device=self.dev)
-            lg = self.logits(hidden[rows])
+            if list(sample_rows) != list(range(hidden.shape[0])):
+                hidden = hidden.index_select(0, self._upload(sample_rows)[0])
+            lg = self.logits(hidden)
             if spec.get("edits"):
                 t0 = StepCtx()
                 t0.out_val = t0.out_idx = torch.empty(n, 1, device=self.dev)
