@@ -76,12 +76,17 @@ struct ChainParams {
 };
 
 // Shared-memory footprint of the staged activations (+ 2 KB of reduction scratch).
-//   bf16 weights: rows(8|16) x (K+8) bf16          int8 weights: two limb planes of M x stride bytes
+//   bf16 weights: M x (K+8) bf16                    int8 weights: two limb planes of M x stride bytes
+// bf16 weights: normalised rows are always staged, others (XGLOBAL) where they take at most 48 KB.  Read from global memory as
+// they are needed they cost a round trip to L2 per eight tiles of weights (a decode step of four layers of width 2048, one row:
+// 379 -> 340 us with the one-row form of stage_bf16).
+constexpr int kStageRows = 48 * 1024;
+TI_HOST_DEVICE bool rows_staged(int xmode, int M, int K) { return xmode == 1 || M * (K + 8) * 2 <= kStageRows; }
 TI_HOST_DEVICE int limb_stride(int kslice) { return kslice + ((64 - (kslice % 128)) + 128) % 128; }
 TI_HOST_DEVICE size_t x_smem_bytes_impl(int wt, int xmode, int M, int K, int kslice) {
   size_t b = 0;
   if (wt == 0) b = (size_t)2 * M * limb_stride(kslice);
-  else if (xmode == 1) b = (size_t)(M > 8 ? 16 : 8) * (K + 8) * 2;
+  else if (rows_staged(xmode, M, K)) b = (size_t)M * (K + 8) * 2;
   return (b + 2048 + 127) / 128 * 128;
 }
 
@@ -415,37 +420,81 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
   __syncthreads();
 }
 
-// bf16-weight path: RMSNorm(1+w) of up to 16 rows into shared memory as bf16.
-TI_DEVICE void stage_bf16_norm(const GemvParams& p, __nv_bfloat16* xs, int xs_stride, float* scratch) {
-  const int tid = threadIdx.x;
-  const int rows = p.M > 8 ? 16 : 8;
+// bf16-weight path: up to 16 rows into shared memory as bf16, RMS-normalised with (1+w) if the product wants that.
+TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride, float* scratch) {
+  const int tid = threadIdx.x, chunks = p.K >> 3, nthreads = blockDim.x;
+  const bool norm = p.xmode == XNORM;
   float* red = scratch;
   float* rrms = scratch + 256;
-  float acc[16];
+  if (p.M == 1 && chunks <= 5 * nthreads) {
+    // one row (batch-1 decode): read once, held in registers between the sum of squares and the store
+    const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
+    uint4 v[5], nw[5];
+    float ss = 0.f;
 #pragma unroll
-  for (int m = 0; m < 16; ++m) acc[m] = 0.f;
-  const int chunks = p.K >> 3;
-  for (int c = tid; c < chunks; c += blockDim.x) {
-#pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      if (m >= p.M) break;
-      const uint4 v = ld_x16(p.x + (size_t)m * p.ldx + c * 8);
-      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[m] += bf16lo(w4[i]) * bf16lo(w4[i]) + bf16hi(w4[i]) * bf16hi(w4[i]);
+    for (int j = 0; j < 5; ++j) {
+      const int c = tid + j * nthreads;
+      v[j] = c < chunks ? ld_x16(p.x + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
+      nw[j] = norm && c < chunks ? ldg_cached16(p.norm_w + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
     }
+    float rr = 1.f;
+    if (norm) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const uint32_t w4[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ss += bf16lo(w4[i]) * bf16lo(w4[i]) + bf16hi(w4[i]) * bf16hi(w4[i]);
+      }
+      ss = warp_sum(ss);
+      if (lane == 0) red[warp] = ss;
+      __syncthreads();
+      float tot = 0.f;
+      for (int w = 0; w < nwarps; ++w) tot += red[w];
+      rr = rsqrtf(tot / (float)p.K + p.eps);
+    }
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const int c = tid + j * nthreads;
+      if (c >= chunks) continue;
+      uint4 o = v[j];
+      if (norm) {
+        const uint32_t a4[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, n4[4] = {nw[j].x, nw[j].y, nw[j].z, nw[j].w};
+        uint32_t r4[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          r4[i] = pack_bf16(bf16lo(a4[i]) * rr * (1.f + bf16lo(n4[i])), bf16hi(a4[i]) * rr * (1.f + bf16hi(n4[i])));
+        o = make_uint4(r4[0], r4[1], r4[2], r4[3]);
+      }
+      *reinterpret_cast<uint4*>(xs + c * 8) = o;
+    }
+    __syncthreads();
+    return;
   }
-  block_row_reduce(acc, p.M, red, rrms, tid, false);
-  if (tid < p.M) rrms[tid] = rsqrtf(rrms[tid] / (float)p.K + p.eps);
-  __syncthreads();
-  for (int c = tid; c < chunks; c += blockDim.x) {
-    const uint4 nw = ldg_cached16(p.norm_w + c * 8);
-    const uint32_t n4[4] = {nw.x, nw.y, nw.z, nw.w};
-    for (int m = 0; m < rows; ++m) {
-      uint4 o = make_uint4(0, 0, 0, 0);
-      if (m < p.M) {
+  if (norm) {
+    float acc[16];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) acc[m] = 0.f;
+    for (int c = tid; c < chunks; c += nthreads) {
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        if (m >= p.M) break;
         const uint4 v = ld_x16(p.x + (size_t)m * p.ldx + c * 8);
-        const uint32_t a4[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[m] += bf16lo(w4[i]) * bf16lo(w4[i]) + bf16hi(w4[i]) * bf16hi(w4[i]);
+      }
+    }
+    block_row_reduce(acc, p.M, red, rrms, tid, false);
+    if (tid < p.M) rrms[tid] = rsqrtf(rrms[tid] / (float)p.K + p.eps);
+    __syncthreads();
+  }
+  for (int c = tid; c < chunks; c += nthreads) {
+    const uint4 nw = norm ? ldg_cached16(p.norm_w + c * 8) : make_uint4(0, 0, 0, 0);
+    const uint32_t n4[4] = {nw.x, nw.y, nw.z, nw.w};
+    for (int m = 0; m < p.M; ++m) {
+      uint4 o = ld_x16(p.x + (size_t)m * p.ldx + c * 8);
+      if (norm) {
+        const uint32_t a4[4] = {o.x, o.y, o.z, o.w};
         const float rr = rrms[m];
         uint32_t r4[4];
 #pragma unroll
@@ -786,7 +835,7 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
       lstride = limb_stride(p.K);
       xl = smem + (size_t)p.M * lstride;
       if (WT == W_INT8) stage_limbs(p, 0, p.K, xh, xl, lstride, scratch);
-      else if (p.xmode == XNORM) stage_bf16_norm(p, xs, p.K + 8, scratch);
+      else if (rows_staged(p.xmode, p.M, p.K)) stage_bf16(p, xs, p.K + 8, scratch);
       if (WT == W_INT8) {
         inv0 = g < p.M ? scratch[288 + g] : 0.f;
         inv1 = g + 8 < p.M ? scratch[288 + g + 8] : 0.f;
@@ -797,7 +846,7 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
     if (lane == 0)                                // keep the ring full
       for (int s = ws.idx - (int)cidx; s < stages; ++s) ws.next(c, widx, W, q, ring_u32, bar0, stages);
 
-    const bool hi = p.M > 8;
+    const bool hi = p.M > 8, staged = rows_staged(p.xmode, p.M, p.K);
     const bool fine = stamp && op <= 1;           // fine-grained stamps of warp 0's last unit of products 0 and 1
     if (fine) p0.dbg[cta * 32 + 24 + 4 * op] = globaltimer_ns();
     const int grp = unit;
@@ -858,7 +907,7 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
               const uint4 wv = lds128(sbuf + u * 512);
               const int k0 = (tile0 + u) * 32;
               uint4 xv, yv = make_uint4(0, 0, 0, 0);
-              if (p.xmode == XNORM) {
+              if (staged) {
                 xv = lds128(xs0 + k0 * 2);
                 if (hi) yv = lds128(xs1 + k0 * 2);
               } else {

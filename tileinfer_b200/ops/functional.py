@@ -360,13 +360,16 @@ def _limb_stride(kslice: int) -> int:
     return kslice + ((64 - (kslice % 128)) + 128) % 128
 
 
+STAGE_ROWS = 48 * 1024      # rows that need no norm are staged for bf16 weights up to this size (must mirror kStageRows)
+
+
 def x_smem_bytes(wt: int, xmode: int, M: int, K: int, kslice: int) -> int:
     """Shared memory the staged activations take (must mirror x_smem_bytes_impl in gemv_w8a16.cu)."""
     b = 0
     if wt == W_INT8:
         b = 2 * M * _limb_stride(kslice)
-    elif xmode == XNORM:
-        b = (16 if M > 8 else 8) * (K + 8) * 2
+    elif xmode == XNORM or M * (K + 8) * 2 <= STAGE_ROWS:
+        b = M * (K + 8) * 2
     return (b + 2048 + 127) // 128 * 128
 
 
