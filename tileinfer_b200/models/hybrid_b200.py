@@ -29,6 +29,7 @@ from .runtime_b200 import DeviceRuntime, StepCtx
 from .weights import ShardSpec, shard_layer
 
 BF16 = torch.bfloat16
+_GEPI = {EPI_STORE: F.GEPI_STORE, EPI_SWIGLU: F.GEPI_SWIGLU, EPI_ROWPAR: F.GEPI_ROWPAR, EPI_F32: F.GEPI_F32}
 
 
 class _Layer:
@@ -103,6 +104,7 @@ class _ModelBase:
         self.launches_per_decode_step = 0
         self._launches = 0
         self._pending, self._pending_wt = [], 0
+        self._limbs = {}                   # limb planes by (rows, k), within one step
         self.chain = os.environ.get("TI_GEMV_CHAIN", "1") != "0"
         self.ll_handoff = os.environ.get("TI_LL_HANDOFF", "1") == "1"
         # every CTA then reads the packets of all ranks (tp x 40 KB per row): worth it for two ranks (measured +2 %),
@@ -310,21 +312,25 @@ class _StepMixin:
         """Many rows (prefill, batched decode): the tcgen05 GEMM.  int8 weights: limb planes of x first
         (RMSNorm fused); bf16 weights: RMSNorm kernel first when the product wants normalised input."""
         self._flush()
-        gepi = {EPI_STORE: F.GEPI_STORE, EPI_SWIGLU: F.GEPI_SWIGLU, EPI_ROWPAR: F.GEPI_ROWPAR, EPI_F32: F.GEPI_F32}[epi]
-        r = None if resid is None else resid[:M]
+        gepi = _GEPI[epi]
+        first = lambda t: t if t is None or t.shape[0] == M else t[:M]  # noqa: E731
+        xs, out, r = first(x), first(out), first(resid)
         if W.wt == F.W_INT8:
-            limbs = F.quant_rows(x[:M], norm_w=norm_w, eps=self.cfg.rms_eps)
-            F.gemm_w8a16(W, limbs, out=out[:M], epi=gepi, resid=r)
+            # the limb planes of products with one k share a buffer within a step: each is read by the next launch only
+            limbs = self._limbs.get((M, W.K))
+            if limbs is None:
+                limbs = self._limbs[M, W.K] = F.Limbs(M, W.K, self.dev)
+            F.quant_rows(xs, norm_w=norm_w, eps=self.cfg.rms_eps, out=limbs)
+            F.gemm_w8a16(W, limbs, out=out, epi=gepi, resid=r)
             self._launches += 2
             return
-        xs = x[:M]
         if norm_w is not None:
             xs = F.rmsnorm(xs, norm_w, self.cfg.rms_eps)
             self._launches += 1
         elif xs.stride(0) != W.K:
             xs = xs.contiguous()
             self._launches += 1
-        F.gemm_bf16(W, xs, out=out[:M], epi=gepi, resid=r)
+        F.gemm_bf16(W, xs, out=out, epi=gepi, resid=r)
         self._launches += 1
 
     def _gemv(self, W: LinearW, x, out, M, *, xmode, epi, norm_w=None, resid=None, ldo=None, out_idx=None):
@@ -372,7 +378,7 @@ class _StepMixin:
         then int8 limb planes or bf16) on the rows while they are still in registers; then the tcgen05 GEMM."""
         pend, self._ar_pending = self._ar_pending, None
         self._flush()
-        gepi = {EPI_STORE: F.GEPI_STORE, EPI_SWIGLU: F.GEPI_SWIGLU, EPI_ROWPAR: F.GEPI_ROWPAR, EPI_F32: F.GEPI_F32}[epi]
+        gepi = _GEPI[epi]
         r = None if resid is None else resid[:M]
         if W.wt == F.W_INT8:
             limbs = F.Limbs(M, W.K, self.dev)
@@ -447,6 +453,7 @@ class _StepMixin:
         F.embed(x.ids, self.embed, x.h[0], self.step_ptr)
         self._launches += 1
         self._order = 0
+        self._limbs = {}
         cur, nxt = x.h[0], x.h[1]
         ig = ia = 0
         for li, L in enumerate(self.layers):
@@ -524,6 +531,7 @@ class _StepMixin:
             cur, nxt = nxt, cur
         self._flush()
         self._ar_flush()
+        self._limbs = {}
         nvtx_end()
         return cur
 

@@ -793,7 +793,7 @@ _GEMM_WS = {}
 def _gemm_workspace(device):
     """Split-k partials (fp32, 32 MB: 16 slices of 128 rows x 4096 columns, or fewer of wider products) and the
     per-tile arrival counters, one set per device; launches on one stream use them one after the other."""
-    key = str(device)
+    key = device.index if isinstance(device, torch.device) else str(device)
     if key not in _GEMM_WS:
         _GEMM_WS[key] = (torch.empty(8 << 20, dtype=torch.float32, device=device),
                          torch.zeros(256, dtype=torch.int32, device=device))

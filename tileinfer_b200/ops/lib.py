@@ -103,7 +103,8 @@ def ptr(t) -> int:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream (without the Stream object that torch.cuda.current_stream builds: 0.5 us a launch, not 8)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def check(rc: int, what: str):
