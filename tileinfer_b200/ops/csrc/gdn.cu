@@ -302,8 +302,9 @@ TI_DEVICE float ld_cluster_f32(const float* local, int rank) {
 // walks ~20 sequences per block one after the other and reaches a third of it).  A warp owns a quarter of the key
 // rows and 32 consecutive columns, so every state access is one full 128-byte line; the two matrix-vector
 // products meet across the four warps in shared memory.  The gated RMSNorm spans the whole head: this kernel writes
-// the un-normalised output and gdn_finish_kernel applies norm * silu(z) in place.  The NSPL blocks of a head form a
-// thread-block cluster (they share the q / k conv history).
+// the un-normalised output and gdn_finish_kernel applies norm * silu(z) in place.  The NSPL blocks of a head read the same
+// q / k conv history; it moves on in gdn_finish_kernel, so that no block waits for another
+// (as a cluster with a barrier between reading and writing: 64 sequences of 48 heads, fp32 states, 104 us against 90).
 template <int DK, int DV, typename ST>
 __global__ void __launch_bounds__(128, sizeof(ST) == 4 ? 8 : 6) gdn_token_split_kernel(const __grid_constant__ GdnParams p) {
   constexpr int CB = 32, NSPL = DV / CB, DPT = DK / 4;
@@ -357,13 +358,12 @@ __global__ void __launch_bounds__(128, sizeof(ST) == 4 ? 8 : 6) gdn_token_split_
       x0[u] = x3;                                          // kept for the history update below
     }
   }
-  // The q / k history of a head is read by all NSPL blocks of the cluster and written by part 0: nobody writes
-  // before every block of the cluster has read (the blocks of a cluster are co-scheduled).
-  cluster_sync_all();
+  // The history of this block's value columns moves on here; that of q and k, which all NSPL blocks of a head read, in
+  // gdn_finish_kernel, once they are done.
 #pragma unroll
   for (int u = 0; u < NCPT; ++u) {
     const int ch = tid + u * 128;
-    if (ch < NCHL && (part == 0 || ch >= 2 * DK)) {
+    if (ch < NCHL && ch >= 2 * DK) {
       cs[hch[u]] = __float2bfloat16_rn(x1[u]);
       cs[NCH + hch[u]] = __float2bfloat16_rn(x2[u]);
       cs[2 * NCH + hch[u]] = __float2bfloat16_rn(x0[u]);
@@ -402,30 +402,62 @@ __global__ void __launch_bounds__(128, sizeof(ST) == 4 ? 8 : 6) gdn_token_split_
   }
 }
 
-// gated RMSNorm over the head * silu(z), in place on the un-normalised output of the split kernel: a warp per
-// (sequence, v-head)
+// After the split kernel: gated RMSNorm over the head * silu(z), in place on its un-normalised output, and the convolution
+// history of q and k.  A warp per (sequence, v-head).
+template <int N> TI_DEVICE void copy_bf16(__nv_bfloat16 (&v)[N], const __nv_bfloat16* p, bool vec) {      // N 2, 4 or 8
+  if (vec) {
+    if constexpr (N == 8) *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(p);
+    else if constexpr (N == 4) *reinterpret_cast<uint2*>(v) = *reinterpret_cast<const uint2*>(p);
+    else *reinterpret_cast<uint32_t*>(v) = *reinterpret_cast<const uint32_t*>(p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = p[i];
+  }
+}
 template <int DK, int DV>
 __global__ void __launch_bounds__(256) gdn_finish_kernel(const __grid_constant__ GdnParams p, int num_seqs) {
-  constexpr int E = DV / 32;
+  constexpr int E = DV / 32, C = 2 * DK / 32, NCH = 2 * DK + DV;      // output columns, q / k channels per lane
   const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   pdl_trigger();
   pdl_wait();
   if (item >= num_seqs * p.hv) return;
   const int s = item / p.hv, vh = item - s * p.hv;
   const int tok = first_token(p, s);
+  const bool vec = p.ld % C == 0 && (reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.conv_state)) % 16 == 0;
+  const __nv_bfloat16* row = p.proj + (size_t)tok * p.ld;
+  // this lane's C channels of [q | k]: rows 1 and 2 of the history and the new input become rows 0, 1 and 2
+  const int kh = vh / (p.hv / p.hk), ch = lane * C, col = ch < DK ? kh * DK + ch : p.hk * DK + kh * DK + (ch - DK);
+  __nv_bfloat16* hist = p.conv_state + ((size_t)p.slots[s] * p.hv + vh) * 3 * NCH + ch;
+  alignas(16) __nv_bfloat16 h[3][C];
+  copy_bf16<C>(h[0], hist + NCH, vec);
+  copy_bf16<C>(h[1], hist + 2 * NCH, vec);
+  copy_bf16<C>(h[2], row + col, vec);
   __nv_bfloat16* o = p.out + (size_t)tok * p.hv * DV + vh * DV + lane * E;
-  const __nv_bfloat16* z = p.proj + (size_t)tok * p.ld + 2 * p.hk * DK + p.hv * DV + vh * DV + lane * E;
+  const __nv_bfloat16* z = row + 2 * p.hk * DK + p.hv * DV + vh * DV + lane * E;
+  alignas(16) __nv_bfloat16 ov[E], zv[E];
+  const bool vec_o = p.ld % E == 0 && (reinterpret_cast<uintptr_t>(p.proj) | reinterpret_cast<uintptr_t>(p.out)) % 16 == 0;
+  copy_bf16<E>(ov, o, vec_o);
+  copy_bf16<E>(zv, z, vec_o);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    if (vec) {
+      if constexpr (C == 8) *reinterpret_cast<uint4*>(hist + j * NCH) = *reinterpret_cast<const uint4*>(h[j]);
+      else *reinterpret_cast<uint2*>(hist + j * NCH) = *reinterpret_cast<const uint2*>(h[j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < C; ++i) hist[j * NCH + i] = h[j][i];
+    }
+  }
   float v[E], ss = 0.f;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    v[e] = __bfloat162float(o[e]);
+    v[e] = __bfloat162float(ov[e]);
     ss += v[e] * v[e];
   }
   ss = warp_sum(ss);
   const float rr = rsqrtf(ss / (float)DV + p.eps);
 #pragma unroll
-  for (int e = 0; e < E; ++e)
-    o[e] = __float2bfloat16_rn(v[e] * rr * p.norm_w[lane * E + e] * silu_f(__bfloat162float(z[e])));
+  for (int e = 0; e < E; ++e) o[e] = __float2bfloat16_rn(v[e] * rr * p.norm_w[lane * E + e] * silu_f(__bfloat162float(zv[e])));
 }
 
 template <int DK, int DV, typename ST, int NS>
@@ -677,26 +709,7 @@ static cudaError_t launch_token(const GdnParams& p, int num_seqs, dim3 grid, cud
 
 template <int DK, int DV, typename ST>
 static cudaError_t launch_token_split(const GdnParams& p, int num_seqs, cudaStream_t st) {
-  constexpr int NSPL = DV / 32;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.hv * NSPL, num_seqs);
-  cfg.blockDim = dim3(128);
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  int n = 0;
-  if (pdl_enabled()) {
-    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
-  }
-  at[n].id = cudaLaunchAttributeClusterDimension;
-  at[n].val.clusterDim.x = NSPL;
-  at[n].val.clusterDim.y = 1;
-  at[n].val.clusterDim.z = 1;
-  ++n;
-  cfg.attrs = at;
-  cfg.numAttrs = n;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gdn_token_split_kernel<DK, DV, ST>, p);
+  const cudaError_t e = launch_kernel(gdn_token_split_kernel<DK, DV, ST>, dim3(p.hv * (DV / 32), num_seqs), dim3(128), 0, st, true, p);
   if (e != cudaSuccess) return e;
   return launch_kernel(gdn_finish_kernel<DK, DV>, dim3((num_seqs * p.hv + 7) / 8), dim3(256), 0, st, true, p, num_seqs);
 }
