@@ -26,6 +26,12 @@
 // vanishes, so the scores of a tile are read once, two threads can share a query row (eight softmax warps, half of the keys
 // of a tile each), and with shared memory for two P tiles the next one is written while P V of this one runs.  Every wait is bounded; on expiry the status word is set, all roles leave their loops
 // and TMEM is freed.  No load carries a cluster-multicast qualifier.
+//
+// PAIR: two heads of one KV head, as a cluster of two CTAs (cta_group::2).  A CTA alone pulls all of K and V through L2 for its
+// 128 query rows, 128 KB per tile of 128 keys at D = 256: as many cycles as the tensor pipe needs for the tile, from single
+// buffers.  A pair's products have M = 256: each CTA holds its own queries, half of the keys of a tile (N of Q K^T) and half of
+// the value columns (N of P V), so half the bytes cross L2 per query, and K and V fit twice.  The first CTA issues all MMAs;
+// `full` barriers are its own and count both CTAs' bytes and softmax threads, `empty` and S barriers are arrived on in both.
 #include "tensor_map.cuh"
 
 namespace ti {
@@ -119,22 +125,28 @@ constexpr float kMaskVal = -1e30f;
 constexpr float kFirstMax = -1e29f;      // a row may see no key of its first tile: its scores are -inf, its weights 0
 constexpr float kRescaleGap = 8.f;       // log2 units the running maximum may lag behind before O is rescaled
 
-template <int D, int DV, int MODE> struct AttnPrefillGeom {
+template <int D, int DV, int MODE, bool PAIR = false> struct AttnPrefillGeom {
   static constexpr int kSlabs = D / 64;
   static constexpr int kQBytes = kSlabs * 128 * 128;
-  static constexpr int kKBytes = kSlabs * 128 * 128;
-  static constexpr int kVPage = DV * 32;
+  static constexpr int kPages = PAIR ? 4 : 8;                       // K pages per tile that this CTA fetches
+  static constexpr int kKBytes = kPages * kSlabs * 2048;
+  static constexpr int kVCols = PAIR ? DV / 2 : DV;                 // value columns that this CTA fetches
+  static constexpr int kVPage = kVCols * 32;
   static constexpr int kVBytes = 8 * kVPage;
   static constexpr int kP = 2 * 128 * 128;                          // one P tile
-  static constexpr int kBarBytes = 128;
-  static constexpr int kPTiles = MODE == SCORE_SERIES && kQBytes + kKBytes + kVBytes + 2 * kP + kBarBytes + 1024 + 1024 <= 227 * 1024 ? 2 : 1;
+  static constexpr int kBarBytes = 128, kExtra = 32 + (PAIR ? 2048 : 0);   // barriers; abort flag, P barriers of the second CTA, exchanged maxima
+  static constexpr int kPTiles = PAIR || (MODE == SCORE_SERIES && kQBytes + kKBytes + kVBytes + 2 * kP + kBarBytes + 1024 + 1024 <= 227 * 1024) ? 2 : 1;
   static constexpr int kPBytes = kPTiles * kP;
-  static constexpr int kStages = kQBytes + 2 * (kKBytes + kVBytes) + kPBytes + kBarBytes + 1024 + 1024 <= 227 * 1024 ? 2 : 1;   // of K and of V
-  static constexpr int kHalves = MODE == SCORE_SERIES ? 2 : 1;      // threads that share a query row
-  static constexpr int kThreads = MODE == SCORE_SERIES ? 384 : kAttnThreads;
-  static constexpr size_t kNeeded = (size_t)kQBytes + kStages * (kKBytes + kVBytes) + kPBytes + kBarBytes + 1024;
+  // tiles of K, and of V (PAIR: one, as two halves)
+  static constexpr int kStages = PAIR || kQBytes + 2 * (kKBytes + kVBytes) + kPBytes + kBarBytes + 1024 + 1024 <= 227 * 1024 ? 2 : 1;
+  static constexpr int kVTotal = (PAIR ? 1 : kStages) * kVBytes;
+  static constexpr int kHalves = PAIR || MODE == SCORE_SERIES ? 2 : 1;     // threads that share a query row
+  static constexpr int kThreads = kHalves == 2 ? 384 : kAttnThreads;
+  // what aligns the tiles to 1024 bytes (PAIR has no room for it: the declared alignment is checked instead)
+  static constexpr size_t kNeeded = (size_t)kQBytes + kStages * kKBytes + kVTotal + kPBytes + kBarBytes + kExtra + (PAIR ? 0 : 1024);
   // one CTA per SM (the kernel takes all 512 TMEM columns)
   static constexpr size_t kSmem = kNeeded > 120 * 1024 ? kNeeded : 120 * 1024;
+  static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
 // What scales a head's output beside 1 / l
@@ -176,24 +188,31 @@ TI_DEVICE void store_rows32(const AttnPrefillParams& p, const uint32_t (&v)[32],
   }
 }
 
-template <int D, int DV, int MODE>
-__global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) attn_prefill_kernel(const __grid_constant__ AttnPrefillParams p) {
-  using G = AttnPrefillGeom<D, DV, MODE>;
+template <int D, int DV, int MODE, bool PAIR>
+__global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads), 1) attn_prefill_kernel(const __grid_constant__ AttnPrefillParams p) {
+  using G = AttnPrefillGeom<D, DV, MODE, PAIR>;
+  constexpr int CTAS = PAIR ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t q_s = smem_u32(smem), k_s = q_s + G::kQBytes, v_s = k_s + G::kStages * G::kKBytes, p_s = v_s + G::kStages * G::kVBytes;
+  const uint32_t q_s = smem_u32(smem), k_s = q_s + G::kQBytes, v_s = k_s + G::kStages * G::kKBytes, p_s = v_s + G::kVTotal;
   const uint32_t bars = p_s + G::kPBytes;
   // two each: k and v one per stage, p one per P tile
   const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56,
                  s_full0 = bars + 72, p_full = bars + 88, p_empty = bars + 104, tmem_slot = bars + 120;
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem + (tmem_slot - q_s));
   constexpr int NP = G::kPTiles, NS = G::kStages;
-  __shared__ int s_abort;
+  int* s_abort = reinterpret_cast<int*>(smem + (bars + G::kBarBytes - q_s));
+  const uint32_t p_local = bars + G::kBarBytes + 16;                      // PAIR, second CTA: its softmax warps are done with P tile 0 / 1
+  float* s_max = reinterpret_cast<float*>(s_abort + 8);                   // PAIR: [tile parity][half][row]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, head = blockIdx.y;
+  const int tile = PAIR ? blockIdx.y : blockIdx.x, head = PAIR ? blockIdx.x : blockIdx.y;      // a pair is two neighbours along x
   const int ntok = p.qt_ntok[tile];
-  if (ntok <= 0) return;                                   // padding tile (uniform over the CTA)
+  if (ntok <= 0) return;                                   // padding tile (uniform over the cluster)
+  if (PAIR && (smem_u32(smem_raw) & 1023) != 0) {
+    if (threadIdx.x == 0) atomicOr(p.status, kStatusBadArgument);
+    return;
+  }
   const int seq = p.qt_seq[tile], tok0 = p.qt_tok0[tile];
   const int kh = head / (p.hq / p.hkv);
   const int kv_len = p.positions[tok0 + ntok - 1] + 1;
@@ -202,24 +221,45 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) a
   const int ntiles = (kv_len - first + 127) >> 7;
 
   if (threadIdx.x == 0) {
-    s_abort = 0;
+    *s_abort = 0;
     mbar_init(q_full, 1);
     for (int i = 0; i < 10; ++i) mbar_init(k_full + 8 * i, 1);       // up to s_full
     for (int i = 0; i < NP; ++i) {
-      mbar_init(p_full + 8 * i, 128 * G::kHalves);
+      mbar_init(p_full + 8 * i, PAIR ? 9 : 128 * G::kHalves);               // PAIR: eight warps, and one arrival for the other CTA's
+      if (PAIR) mbar_init(p_local + 8 * i, 8);
       mbar_init(p_empty + 8 * i, 1);
     }
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(tmem_slot, 512);
+    } else {
+      tmem_alloc(tmem_slot, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  volatile int* abort_flag = &s_abort;
+  volatile int* abort_flag = s_abort;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  auto lead = [&](uint32_t bar) { return PAIR ? map_to_rank(bar, 0) : bar; };       // the first CTA's barrier
+  auto expect = [&](uint32_t bar, uint32_t bytes) { if (rank == 0) mbar_expect_tx(bar, CTAS * bytes); };
+  auto load_2d = [&](uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    if (PAIR) tma_pair_2d(dst, map, c0, c1, bar);
+    else tma_load_2d(dst, map, c0, c1, bar);
+  };
+  auto commit = [&](uint32_t bar) {
+    if (PAIR) umma_commit_pair(bar);
+    else umma_commit(bar);
+  };
+  auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    if (PAIR) umma_pair_bf16(d, a, b, idesc, acc);
+    else umma_bf16(d, a, b, idesc, acc);
+  };
 
   if (warp == 0 || warp == kAttnProducerV) {
     // ------------------------------------------------------------ TMA producers: warp 0 Q and K, warp 6 V
@@ -228,47 +268,56 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) a
     if (elect_one()) {
       const int* bt = p.block_tables + (size_t)seq * p.max_blocks;
       if (warp == 0) {
-        mbar_expect_tx(q_full, G::kQBytes);
+        expect(q_full, G::kQBytes);
+        const uint32_t q_of = lead(q_full), k_of = lead(k_full);
 #pragma unroll
-        for (int s = 0; s < G::kSlabs; ++s) tma_load_2d(q_s + s * (128 * 128), &p.map_q, head * D + s * 64, tok0, q_full);
+        for (int s = 0; s < G::kSlabs; ++s) load_2d(q_s + s * (128 * 128), &p.map_q, head * D + s * 64, tok0, q_of);
         for (int j = 0; j < ntiles && !*abort_flag; ++j) {
-          int blk[8];
+          int blk[G::kPages];
 #pragma unroll
-          for (int g = 0; g < 8; ++g) blk[g] = bt[min(page0 + j * 8 + g, npages - 1)];   // pages past the end repeat the last one (masked)
+          for (int g = 0; g < G::kPages; ++g) blk[g] = bt[min(page0 + j * 8 + (int)rank * G::kPages + g, npages - 1)];   // pages past the end repeat the last one (masked)
           const int st = j % NS;
           if (j >= NS && !mbar_wait(k_empty + 8 * st, (uint32_t)((j / NS - 1) & 1), kAttnWaitNs, p.status)) { *abort_flag = 1; break; }
-          mbar_expect_tx(k_full + 8 * st, G::kKBytes);
+          expect(k_full + 8 * st, G::kKBytes);
 #pragma unroll
-          for (int g = 0; g < 8; ++g)
-            tma_load_4d(k_s + st * G::kKBytes + g * (G::kSlabs * 2048), &p.map_k, 0, 0, 0, (blk[g] * p.hkv + kh) * 2, k_full + 8 * st);
+          for (int g = 0; g < G::kPages; ++g) {
+            const uint32_t dst = k_s + st * G::kKBytes + g * (G::kSlabs * 2048);
+            if (PAIR) tma_pair_4d(dst, &p.map_k, 0, 0, 0, (blk[g] * p.hkv + kh) * 2, k_of + 8 * st);
+            else tma_load_4d(dst, &p.map_k, 0, 0, 0, (blk[g] * p.hkv + kh) * 2, k_of + 8 * st);
+          }
         }
       } else {
-        for (int j = 0; j < ntiles && !*abort_flag; ++j) {
-          int blk[8];
+        // PAIR: a stage is half a tile (four pages), so that the first half of the next tile can be fetched while P V works on
+        // the second half of this one
+        constexpr int HV = PAIR ? 2 : 1, PG = 8 / HV, NSV = PAIR ? 2 : NS;
+        const uint32_t v_of = lead(v_full);
+        for (int i = 0; i < HV * ntiles && !*abort_flag; ++i) {
+          int blk[PG];
 #pragma unroll
-          for (int g = 0; g < 8; ++g) blk[g] = bt[min(page0 + j * 8 + g, npages - 1)];
-          const int st = j % NS;
-          if (j >= NS && !mbar_wait(v_empty + 8 * st, (uint32_t)((j / NS - 1) & 1), kAttnWaitNs, p.status)) { *abort_flag = 1; break; }
-          mbar_expect_tx(v_full + 8 * st, G::kVBytes);
+          for (int g = 0; g < PG; ++g) blk[g] = bt[min(page0 + i * PG + g, npages - 1)];
+          const int st = i % NSV;
+          if (i >= NSV && !mbar_wait(v_empty + 8 * st, (uint32_t)((i / NSV - 1) & 1), kAttnWaitNs, p.status)) { *abort_flag = 1; break; }
+          expect(v_full + 8 * st, PG * G::kVPage);
 #pragma unroll
-          for (int g = 0; g < 8; ++g) tma_load_2d(v_s + st * G::kVBytes + g * G::kVPage, &p.map_v, 0, (blk[g] * p.hkv + kh) * DV, v_full + 8 * st);
+          for (int g = 0; g < PG; ++g)
+            load_2d(v_s + (st * PG + g) * G::kVPage, &p.map_v, 0, (blk[g] * p.hkv + kh) * DV + (int)rank * G::kVCols, v_of + 8 * st);
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
-      constexpr uint32_t idesc_s = idesc_f16_bf16(128, 128), idesc_o = idesc_f16_bf16(128, DV);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc_s = idesc_f16_bf16(128 * CTAS, 128), idesc_o = idesc_f16_bf16(128 * CTAS, DV);
       auto issue_qk = [&](int j) {
         const uint32_t d = tmem_base + (uint32_t)(j & 1) * 128u, kb = k_s + (j % NS) * G::kKBytes;
 #pragma unroll
         for (int s = 0; s < G::kSlabs; ++s)
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)                     // K: per 8-key group the kSlabs 64-column slabs side by side
-            umma_bf16(d, smem_desc_sw128(q_s + s * (128 * 128) + ks * 32),
+            mma(d, smem_desc_sw128(q_s + s * (128 * 128) + ks * 32),
                       smem_desc_sw128_sbo(kb + s * 1024 + ks * 32, G::kSlabs * 1024), idesc_s, (s | ks) ? 1u : 0u);
-        umma_commit(k_empty + 8 * (j % NS));
-        umma_commit(s_full0 + 8 * (j & 1));
+        commit(k_empty + 8 * (j % NS));
+        commit(s_full0 + 8 * (j & 1));
       };
       bool ok = mbar_wait(q_full, 0, kAttnWaitNs, p.status) && mbar_wait(k_full, 0, kAttnWaitNs, p.status);
       if (ok) {
@@ -282,17 +331,35 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) a
           tc_fence_after();
           issue_qk(j + 1);
         }
-        ok = mbar_wait(p_full + 8 * (j % NP), (uint32_t)((j / NP) & 1), kAttnWaitNs, p.status) && mbar_wait(v_full + 8 * (j % NS), (uint32_t)((j / NS) & 1), kAttnWaitNs, p.status);
-        if (!ok) break;
-        tc_fence_after();
+        ok = PAIR ? mbar_wait_cluster(p_full + 8 * (j % NP), (uint32_t)((j / NP) & 1), kAttnWaitNs, p.status)
+                  : mbar_wait(p_full + 8 * (j % NP), (uint32_t)((j / NP) & 1), kAttnWaitNs, p.status);
+        constexpr int HV = PAIR ? 2 : 1, PG = 8 / HV, NSV = PAIR ? 2 : NS;
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
-          umma_bf16(tmem_base + 256u, smem_desc_sw128(p_s + (j % NP) * G::kP + (g >> 2) * (128 * 128) + (g & 3) * 32),
-                    smem_desc_sw32(v_s + (j % NS) * G::kVBytes + g * G::kVPage), idesc_o, (j | g) ? 1u : 0u);
-        umma_commit(v_empty + 8 * (j % NS));
-        umma_commit(p_empty + 8 * (j % NP));
+        for (int h = 0; h < HV; ++h) {
+          const int i = HV * j + h, st = i % NSV;
+          ok = ok && mbar_wait(v_full + 8 * st, (uint32_t)((i / NSV) & 1), kAttnWaitNs, p.status);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int gg = 0; gg < PG; ++gg) {
+            const int g = h * PG + gg;
+            mma(tmem_base + 256u, smem_desc_sw128(p_s + (j % NP) * G::kP + (g >> 2) * (128 * 128) + (g & 3) * 32),
+                smem_desc_sw32(v_s + (st * PG + gg) * G::kVPage), idesc_o, (j | g) ? 1u : 0u);
+          }
+          commit(v_empty + 8 * st);
+        }
+        if (!ok) break;
+        commit(p_empty + 8 * (j % NP));
       }
       if (!ok) *abort_flag = 1;
+    } else if (PAIR && rank == 1 && elect_one()) {
+      // the second CTA's softmax warps arrive here and one remote arrival is passed on: a release at cluster scope stalls the
+      // warp that makes it (a fifth of the softmax warps' time when each made its own)
+      const uint32_t p_of = lead(p_full);
+      for (int j = 0; j < ntiles && !*abort_flag; ++j) {
+        if (!mbar_wait(p_local + 8 * (j & 1), (uint32_t)((j >> 1) & 1), kAttnWaitNs, p.status)) { *abort_flag = 1; break; }
+        mbar_arrive_cluster(p_of + 8 * (j & 1));
+      }
     }
   } else if (MODE == SCORE_SERIES) {
     // ------------------------------------------------------------ softmax + epilogue, bounded scores: two threads (in
@@ -363,6 +430,131 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) a
         const size_t tok = (size_t)tok0 + (valid ? r : 0);
         const float inv = head_factor(p, tok, head) / (l_s[r] + l_s[128 + r]);
         const __nv_bfloat16* gate = p.gate_src + tok * p.ld + p.gate_col + (size_t)head * p.gate_stride;
+        __nv_bfloat16* dst = p.out + tok * (size_t)p.ldo + (size_t)head * DV;
+#pragma unroll 1
+        for (int c = half * (DV / 64); c < (half + 1) * (DV / 64); ++c) {
+          uint32_t v[32];
+          tmem_ld32(lane_base + 256u + c * 32, v);
+          uint4 gates[4];
+          load_gates(p, gate, c, gates);
+          tmem_ld_wait();
+          if (valid) store_rows32(p, v, inv, gates, dst, c);
+        }
+      }
+      tc_fence_before();
+    }
+  } else if (PAIR) {
+    // ------------------------------------------------------------ softmax + epilogue: two threads (in warps 2-5 and 8-11) per
+    // query row, each half of the keys of a tile and half of the output columns.  A warp whose wait ran out goes on through
+    // the named barriers, which both warps of a row have to reach.
+    if (warp < 6 || warp >= 8) {
+      const int quarter = warp & 3, half = warp >= 8 ? 1 : 0, r = quarter * 32 + lane;
+      const bool valid = r < ntok;
+      const int pos = p.positions[tok0 + (valid ? r : ntok - 1)];
+      const int lo = p.window > 0 ? pos - p.window + 1 : 0;
+      const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      const size_t tok = (size_t)tok0 + (valid ? r : 0);
+      const __nv_bfloat16* gate = p.gate_src + tok * p.ld + p.gate_col + (size_t)head * p.gate_stride;
+      prefetch_gates(p, gate + half * (DV / 2), DV / 2);
+      const uint32_t p_done = rank == 0 ? p_full : p_local;
+      float m_used = kFirstMax, l = 0.f;
+      bool ok = true;
+      for (int j = 0; j < ntiles; ++j) {
+        ok = ok && !*abort_flag && mbar_wait(s_full0 + 8 * (j & 1), (uint32_t)((j >> 1) & 1), kAttnWaitNs, p.status);
+        ok = __all_sync(0xffffffffu, ok);
+        uint32_t v[2][32];
+        float mx = __uint_as_float(0xff800000u);
+        if (ok) {
+          tc_fence_after();
+          const uint32_t s_addr = lane_base + (uint32_t)(j & 1) * 128u + (uint32_t)half * 64u;
+          const int key0 = first + j * 128 + half * 64, from = lo - key0, to = pos - key0;     // the row sees keys from .. to of its half
+          tmem_ld32(s_addr, v[0]);
+          tmem_ld32(s_addr + 32, v[1]);
+          tmem_ld_wait();
+          if (to < 63 || from > 0) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (c * 32 + i > to || c * 32 + i < from) v[c][i] = 0xff800000u;
+          }
+          float m4[4] = {mx, mx, mx, mx};
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(v[c][i]));
+          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+        }
+        float* sm = s_max + (j & 1) * 256;                  // written again two tiles on, after the next barrier
+        sm[half * 128 + r] = mx;
+        asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quarter) : "memory");       // the two warps of these rows
+        if (!ok) continue;
+        mx = fmaxf(mx, sm[(half ^ 1) * 128 + r]) * p.scale_log2e;
+        const float m_new = fmaxf(m_used, mx);              // the same in both threads of the row
+        const bool resc = m_new - m_used > kRescaleGap;
+        float alpha = 1.f;
+        if (resc) {
+          alpha = ex2_approx(m_used - m_new);
+          l *= alpha;
+          m_used = m_new;
+        }
+        // ---- the P tile is free once P V of two tiles ago has completed; O is quiescent once that of the last tile has
+        if (j >= 2) ok = mbar_wait(p_empty + 8 * (j & 1), (uint32_t)(((j >> 1) - 1) & 1), kAttnWaitNs, p.status);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) continue;
+        if (j > 0 && __any_sync(0xffffffffu, resc)) {
+          ok = mbar_wait(p_empty + 8 * ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1), kAttnWaitNs, p.status);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) continue;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = half * (DV / 64); c < (half + 1) * (DV / 64); ++c) {
+            uint32_t o[32];
+            tmem_ld32(lane_base + 256u + c * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st32(lane_base + 256u + c * 32, o);
+          }
+          tmem_st_wait();
+        }
+        // ---- P = exp2(S - m), row sum, bf16 A operand in the 128-byte-swizzled K-major layout
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t row_addr = p_s + (uint32_t)(j & 1) * G::kP + (uint32_t)half * (128 * 128) + (uint32_t)r * 128u;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float p0 = ex2_approx(fmaf(__uint_as_float(v[c][i]), p.scale_log2e, -m_used)), p1 = ex2_approx(fmaf(__uint_as_float(v[c][i + 1]), p.scale_log2e, -m_used));
+            s4[(i >> 1) & 3] += p0 + p1;
+            pk[i >> 1] = pack_bf16(p0, p1);
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const uint32_t chunk = (uint32_t)(c * 4 + q4) ^ (uint32_t)(r & 7);
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(row_addr + chunk * 16u), "r"(pk[4 * q4]),
+                         "r"(pk[4 * q4 + 1]), "r"(pk[4 * q4 + 2]), "r"(pk[4 * q4 + 3])
+                         : "memory");
+          }
+        }
+        l += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        tc_fence_before();
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(p_done + 8 * (j & 1)) : "memory");
+      }
+      if (ok) {                                            // every P V has completed: they complete in order
+        ok = mbar_wait(p_empty + 8 * ((ntiles - 1) & 1), (uint32_t)(((ntiles - 1) >> 1) & 1), kAttnWaitNs, p.status);
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      if (!ok) *abort_flag = 1;
+      float* sm = s_max + (ntiles & 1) * 256;
+      sm[half * 128 + r] = l;
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quarter) : "memory");
+      if (ok) {
+        tc_fence_after();
+        const float inv = head_factor(p, tok, head) / (l + sm[(half ^ 1) * 128 + r]);
         __nv_bfloat16* dst = p.out + tok * (size_t)p.ldo + (size_t)head * DV;
 #pragma unroll 1
         for (int c = half * (DV / 64); c < (half + 1) * (DV / 64); ++c) {
@@ -503,26 +695,49 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE>::kThreads), 1) a
     tc_fence_before();
   }
   __syncthreads();
+  if (PAIR) cluster_sync_all();                            // neither CTA leaves while the other may use its memory
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
 }
 
-template <int D, int DV, int MODE>
+template <int D, int DV, int MODE, bool PAIR = false>
 static int launch_mode(const AttnPrefillParams& p, int num_tiles, cudaStream_t st) {
+  using G = AttnPrefillGeom<D, DV, MODE, PAIR>;
   static bool configured = false;
-  auto k = attn_prefill_kernel<D, DV, MODE>;
+  auto k = attn_prefill_kernel<D, DV, MODE, PAIR>;
   if (!configured) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AttnPrefillGeom<D, DV, MODE>::kSmem);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
     configured = true;
   }
-  k<<<dim3(num_tiles, p.hq), AttnPrefillGeom<D, DV, MODE>::kThreads, AttnPrefillGeom<D, DV, MODE>::kSmem, st>>>(p);
-  return (int)cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = PAIR ? dim3(p.hq, num_tiles) : dim3(num_tiles, p.hq);
+  cfg.blockDim = dim3(G::kThreads);
+  cfg.dynamicSmemBytes = G::kSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// Pairs of CTAs: plain scores of heads of 128 or 256 values, where neighbouring heads share their keys and values (the figures
+// above; other heads and scores have one form only).  Tiles are the grid's second dimension.
+static bool attn_pair(int hq, int hkv, int D, int DV, int mode, int num_tiles) {
+  return mode == SCORE_PLAIN && D == DV && D >= 128 && (hq / hkv) % 2 == 0 && num_tiles <= 65535;
 }
 
 template <int D, int DV>
 static int launch_attn_prefill(const AttnPrefillParams& p, int num_tiles, int mode, cudaStream_t st) {
+  if constexpr (D == DV && D >= 128)
+    if (attn_pair(p.hq, p.hkv, D, DV, mode, num_tiles)) return launch_mode<D, DV, SCORE_PLAIN, true>(p, num_tiles, st);
   if (mode == SCORE_SERIES) return launch_mode<D, DV, SCORE_SERIES>(p, num_tiles, st);
   if (mode == SCORE_CAPPED) return launch_mode<D, DV, SCORE_CAPPED>(p, num_tiles, st);
   if (mode == SCORE_BIASED) return launch_mode<D, DV, SCORE_BIASED>(p, num_tiles, st);
@@ -565,7 +780,8 @@ int ti_attn_prefill(const void* q, int T, const void* kcache, const void* vcache
   if (rc) return rc;
   rc = ti::bf16_map_groups(&p.map_k, kcache, D, (long long)num_blocks * hkv * 16, D / 64, 2);
   if (rc) return rc;
-  rc = ti::bf16_map_2d(&p.map_v, vcache, 16, (long long)num_blocks * hkv * DV, 16, DV, CU_TENSOR_MAP_SWIZZLE_32B);
+  const bool pair = ti::attn_pair(hq, hkv, D, DV, mode, num_tiles);
+  rc = ti::bf16_map_2d(&p.map_v, vcache, 16, (long long)num_blocks * hkv * DV, 16, pair ? DV / 2 : DV, CU_TENSOR_MAP_SWIZZLE_32B);
   if (rc) return rc;
   p.block_tables = (const int*)block_tables;
   p.positions = (const int*)positions;
