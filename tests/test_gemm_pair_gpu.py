@@ -1,4 +1,4 @@
-"""The persistent products of many tokens (pairs of CTAs): edges of tiles in every direction, odd numbers of tiles, half
+"""The persistent products (pairs of CTAs): edges of tiles in every direction, odd numbers of tiles, half
 stages of k, every epilogue that stores through another path, against fp64 products of the same operands."""
 import pytest
 import torch
@@ -8,9 +8,12 @@ BF16 = torch.bfloat16
 
 # (tokens, weight rows, k): the last token / weight tile full, one short, one over; fewer k stages than the ring holds;
 # k with a half stage; more tiles than pairs of SMs, not a multiple of them; a last round cut along k in two to four slices,
-# the last slice shorter; nothing but cut tiles
+# the last slice shorter; nothing but cut tiles; tiles of 32 and 64 tokens, full, nearly empty and one over; a short k with many
+# tiles; the last batch of bf16 decodes with one tile per CTA and the first on pairs
 SHAPES = [(256, 16384, 512), (129, 16480, 576), (257, 19200, 320), (4095, 1000, 1152), (2176, 2568, 64), (1060, 5120, 4160),
-          (3000, 1160, 128), (8200, 520, 2048), (128, 5120, 17408), (70, 5128, 8256), (200, 4096, 6144), (1300, 5120, 6144)]
+          (3000, 1160, 128), (8200, 520, 2048), (128, 5120, 17408), (70, 5128, 8256), (200, 4096, 6144), (1300, 5120, 6144),
+          (1, 2048, 2048), (5, 5120, 6144), (17, 16480, 5120), (32, 5120, 17408), (33, 5120, 17408), (50, 1000, 4096), (64, 34816, 2048),
+          (64, 30976, 320), (8, 34816, 1024), (9, 34816, 1024)]
 
 
 def _operands(M, N, K, quantize):

@@ -1,6 +1,6 @@
 // W8A16 GEMM: y[M, N] = x[M, K] * W[N, K]^T on the 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators in tensor
-// memory), fed by TMA.  One output tile per CTA: batched decode, short products and experts; products of many tokens run on
-// pairs of CTAs (gemm_pair.cuh, which shares the operand layouts and epilogues).
+// memory), fed by TMA.  One output tile per CTA: short products, bf16 products of a few tokens, routers and experts; all others run on pairs of CTAs
+// (gemm_pair.cuh, which shares the operand layouts and epilogues).
 //
 // Replaces the reference's M > 1 path, which re-materialises a bf16 copy of the whole int8 weight on every
 // call and hands it to cuBLAS (kernels/splitk_gemv.py:243-247).
@@ -578,12 +578,6 @@ static int launch_gemm(const GemmParams& p, dim3 grid, cudaStream_t st) {
   const cudaError_t e = launch_kernel(k, grid, dim3(kGemmThreads), GemmGeom<BN, BF16, BMH, RK>::kSmem, st, true, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
-
-// 256-row tiles for few tokens: the limb planes are as many bytes per stage as the weights of a 128-row tile; with 256 rows
-// they are half.  That pays only where no k split follows from halving the number of tiles.  Measured at 64 tokens on the 27B
-// shapes (us, 128-row -> 256-row tiles): gate_up 43.6 -> 37.6 (136 tiles, no split), in_proj 23 -> 49 (65 tiles in two k
-// slices), down 47 -> 80, out_proj 36 -> 71.
-static int pick_bmh(int M, int n_tiles) { return M <= 64 && (n_tiles * 8 + 255) / 256 * ((M + 127) / 128) >= 120 ? 2 : 1; }
 
 // k split that fills the 148 SMs when there are few output tiles; sets kb_per_split.  KB counts stages of 128 bytes
 // of k; a slice has at least 16 of them (TI_GEMM_SPLIT_STAGES).  Measured at 64 tokens on N = 5120 (us): K = 6144

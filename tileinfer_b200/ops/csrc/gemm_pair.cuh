@@ -3,8 +3,9 @@
 // The one-tile-per-CTA kernel (gemm_kernel.cuh) is not bound by a pipe at many tokens: tensor pipe 61 % active at 2048 tokens
 // on 34816 x 5120, shared-memory reads 30 %, L2 to SM 29 % (int8) and 43 % (bf16) of their peaks.  What is missing is
 // overlap: filling the ring, the epilogue and the launch of the next CTA stand between two main loops.  Here
-//   * a pair of CTAs owns a tile of 256 weight rows x NT tokens.  One tcgen05.mma of M = 256 reads 128 weight rows and half of
-//     the tokens from each CTA's shared memory, so a CTA fetches 32 KB per 128 bytes of k for 128 x 256 accumulator columns;
+//   * a pair of CTAs owns a tile of 256 weight rows x NT tokens (32 or 64 in batched decode).  One tcgen05.mma of M = 256 reads
+//     128 weight rows and half of the tokens from each CTA's shared memory, so a CTA fetches 32 KB per 128 bytes of k for 128 x
+//     256 accumulator columns;
 //   * the accumulators (256 TMEM columns: NT = 256 tokens of a bf16 product, or two limbs of NT = 128 tokens of an int8 one)
 //     are double-buffered: the epilogue of a tile runs beside the main loop of the next one;
 //   * the ring of stages runs on across tiles.
@@ -315,7 +316,8 @@ struct PairPlan {
 // Cutting the tiles of the last round along k costs a round trip of partial results through L2, about as long as 40 stages,
 // so it has to save 66 stages (128 bytes of k) of that round.  N = 5120, us without / with: K = 17408 int8 (136 stages) at
 // 128 tokens 50 / 35, 512 tokens 88 / 74, 1060 tokens 136 / 130; bf16 (272 stages) 61 / 47, 100 / 91, 185 / 165.  K = 6144 int8
-// (48 stages) at 128 tokens 23.3 / 24.9, 1060 tokens 53 / 57: not cut.
+// (48 stages) at 128 tokens 23.3 / 24.9, 1060 tokens 53 / 57: not cut.  Tiles of 32 and 64 tokens carry a quarter or half of
+// the partial results through L2 and are bound by the weights' arrival, which a cut shares among more SMs: 30 stages.
 static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
   PairPlan q;
   const int tiles = (n_tiles * 8 + 255) / 256 * ((M + NT - 1) / NT);
@@ -323,7 +325,7 @@ static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
   q.slices = q.cut == 0 || !may_cut ? 1 : std::max(1, std::min(std::min(kPairs / q.cut, KS / 16), 8));
   q.kb_per_split = (KS + q.slices - 1) / q.slices;
   q.slices = (KS + q.kb_per_split - 1) / q.kb_per_split;       // no empty slice
-  if (KS - q.kb_per_split < 66) q.slices = 1;
+  if (KS - q.kb_per_split < (NT <= 64 ? 30 : 66)) q.slices = 1;
   if (q.slices == 1) q.cut = 0;
   q.whole = tiles - q.cut;
   q.rounds = (q.whole + kPairs - 1) / kPairs + (q.cut ? (float)q.kb_per_split / KS : 0.f);
@@ -333,18 +335,30 @@ static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
 static bool pair_may_cut(const void* part, size_t part_bytes, const void* tile_count, int n_count) {
   return part != nullptr && tile_count != nullptr && part_bytes >= (size_t)kPairs * 256 * 256 * 4 && n_count >= kPairs;
 }
-// Tokens of a pair's tile of a bf16 product: 128-token tiles cost 0.62 of 256-token ones (34816 x 5120 at 4096 tokens: 1143 us
-// against 917), but leave fewer pairs idle in the last round (5120 x 6144 at 4096 tokens: 221 against 257).
-static int pair_tokens_bf16(int M, int n_tiles, int KS, bool may_cut) {
-  return M <= 128 || 0.62f * pair_plan(M, n_tiles, KS, 128, may_cut).rounds < pair_plan(M, n_tiles, KS, 256, may_cut).rounds ? 128 : 256;
+// Tokens of a pair's tile.  Batched decode: as few as hold the batch.  bf16 products of many tokens: 128-token tiles cost 0.62 of
+// 256-token ones (34816 x 5120 at 4096 tokens: 1143 us against 917), but leave fewer pairs idle in the last round (5120 x 6144 at
+// 4096 tokens: 221 against 257).
+static int pair_tokens(bool bf16, int M, int n_tiles, int KS, bool may_cut) {
+  if (M <= 64) return M <= 32 ? 32 : 64;
+  if (!bf16 || M <= 128) return 128;
+  return 0.62f * pair_plan(M, n_tiles, KS, 128, may_cut).rounds < pair_plan(M, n_tiles, KS, 256, may_cut).rounds ? 128 : 256;
 }
-// Which products the pairs take.  One tile per CTA -> pairs, us, on N x K: 34816 x 5120 at 128 / 1060 / 4096 tokens int8 56 -> 39,
-// 327 -> 239, 1085 -> 810, bf16 70 -> 62, 379 -> 298, 1238 -> 917; 5120 x 6144 int8 30 -> 27, 95 -> 60, 366 -> 186; 2048 x 2048 at 128 /
-// 1060 tokens int8 18 -> 13, 19 -> 15; 1024 x 5120 at 70 tokens 23 -> 18.  The launch of a pair and its first ring fill take
-// about 4 us longer: few tokens with a short k stay (8192 x 512 at 70 tokens 11.1 against 14.5, at 250 15.8 / 15.3, at 512 28.8 ->
-// 16.8), as do products of up to 64 tokens, whose token tiles are smaller (64 tokens of 16480 x 5120: 18.9 against 20.3), and
-// a single tile of weight rows (routers), which would leave half of each pair idle.
-static bool pair_serves(int M, int N, int KS) { return M > 64 && N > 128 && (KS >= 16 || M > 256); }
+// Products with tiles enough for every SM without a k split.
+static bool pair_many(int M, int n_tiles) { return (n_tiles * 8 + 255) / 256 * ((M + 127) / 128) >= 120; }
+// Which products the pairs take.  Not
+//   * short ones, unless they have many tiles: the launch of a pair and its first ring fill take about 4 us longer (8192 x 512 at 70
+//     tokens 11.1 us on one CTA per tile against 14.5, at 250 15.8 / 15.3, at 512 28.8 -> 16.8);
+//   * a single tile of weight rows (routers), which would leave half of each pair idle;
+//   * bf16 products of up to 8 tokens, where weights alone are streamed, twice as many bytes as in int8 (5120 x 17408 at 4 tokens 33.3
+//     us against 35.7, a step of 3 decodes 757 / 763; at 14 decodes 841 -> 827, at 32 934 -> 908).
+// One tile per CTA -> pairs, us, on N x K: 34816 x 5120 at 64 / 128 / 1060 / 4096 tokens int8 37.8 -> 34.0, 56 -> 39, 327 -> 239,
+// 1085 -> 810, bf16 61 -> 61, 70 -> 62, 379 -> 298, 1238 -> 917; 5120 x 17408 at 64 tokens int8 28.2 -> 24.9, bf16 43.2 -> 40.9;
+// 5120 x 6144 int8 18.9 -> 16.1, 30 -> 27, 95 -> 60, 366 -> 186; 2048 x 2048 at 64 / 128 / 1060 tokens int8 12.2 -> 9.6, 18 -> 13, 19 -> 15.
+// At 4 tokens an int8 product alone gains nothing (18.5 -> 17.7, 10.6 -> 11.3, 8.9 -> 9.8), a decode step does, since the next
+// product's weights are requested earlier: 2 decodes of the 27B layers 551 -> 515 us, 5 599 -> 557, 12 652 -> 591, 64 1038 -> 976.
+static bool pair_serves(bool bf16, int M, int n_tiles, int N, int KS) {
+  return N > 128 && !(bf16 && M <= 8) && (KS >= 16 || M > 256 || pair_many(M, n_tiles));
+}
 
 static void pair_apply(GemmParams& p, const PairPlan& q, int n_tiles, int NT, void* part, void* tile_count) {
   p.tiles_n = (n_tiles * 8 + 255) / 256;

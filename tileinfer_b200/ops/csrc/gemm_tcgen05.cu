@@ -184,14 +184,13 @@ int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, 
   const int KB = K / 64, KS = (KB + ti::kKS - 1) / ti::kKS;      // 64-byte slabs of the weight layout; 128-byte stages
   const int BN = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
   const bool may_cut = ti::pair_may_cut(part, part_bytes, tile_count, n_count);
-  const ti::PairPlan plan = ti::pair_plan(M, n_tiles, KS, 128, may_cut);
-  const bool pair = ti::pair_serves(M, N, KS);
-  const int BMH = pair ? 1 : ti::pick_bmh(M, n_tiles);
-  int rc = ti::cached_map(&p.map_w, w, KB, n_tiles, BMH == 2 ? -32 : 0);
+  const bool pair = ti::pair_serves(false, M, n_tiles, N, KS);
+  const int NT = ti::pair_tokens(false, M, n_tiles, KS, may_cut);
+  int rc = ti::cached_map(&p.map_w, w, KB, n_tiles, 0);
   if (rc) return rc;
-  rc = ti::cached_map(&p.map_xh, xh, K, M, pair ? 64 : BN);
+  rc = ti::cached_map(&p.map_xh, xh, K, M, pair ? NT / 2 : BN);
   if (rc) return rc;
-  rc = ti::cached_map(&p.map_xl, xl, K, M, pair ? 64 : BN);
+  rc = ti::cached_map(&p.map_xl, xl, K, M, pair ? NT / 2 : BN);
   if (rc) return rc;
   p.xscale = (const float*)xscale;
   p.wscale = (const __nv_bfloat16*)wscale;
@@ -207,15 +206,13 @@ int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, 
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (pair) {
-    ti::pair_apply(p, plan, n_tiles, 128, part, tile_count);
-    return ti::launch_pair<128, false>(p, st);
+    ti::pair_apply(p, ti::pair_plan(M, n_tiles, KS, NT, may_cut), n_tiles, NT, part, tile_count);
+    if (NT == 32) return ti::launch_pair<32, false>(p, st);
+    return NT == 64 ? ti::launch_pair<64, false>(p, st) : ti::launch_pair<128, false>(p, st);
   }
-  const int rows = ti::kBM * BMH;
-  const int tiles_n = (n_tiles * 8 + rows - 1) / rows, tiles_m = (M + BN - 1) / BN;
+  const int tiles_n = (n_tiles * 8 + ti::kBM - 1) / ti::kBM, tiles_m = (M + BN - 1) / BN;
   const int S = ti::plan_split(p, KS, tiles_n * tiles_m, M, N, ldo, part, part_bytes, tile_count, n_count);
   dim3 grid(tiles_m, tiles_n, S);
-  if (BMH == 2 && BN == 32) return ti::launch_gemm<32, false, 2>(p, grid, st);
-  if (BMH == 2 && BN == 64) return ti::launch_gemm<64, false, 2>(p, grid, st);
   if (BN == 32) return ti::launch_gemm<32, false>(p, grid, st);
   if (BN == 64) return ti::launch_gemm<64, false>(p, grid, st);
   return ti::launch_gemm<128, false>(p, grid, st);
@@ -233,10 +230,11 @@ int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M,
   // a single weight tile (a router): smaller token tiles, so that there are enough of them for all SMs
   const int BN = M <= 32 || (N <= 128 && M <= 64 * 148) ? 32 : (M <= 64 || N <= 128 ? 64 : 128);
   const bool may_cut = ti::pair_may_cut(part, part_bytes, tile_count, n_count);
-  const int NT = ti::pair_tokens_bf16(M, n_tiles, KS, may_cut);
-  const ti::PairPlan plan = ti::pair_plan(M, n_tiles, KS, NT, may_cut);
-  const bool pair = ti::pair_serves(M, N, KS);
-  const int BMH = pair ? 1 : ti::pick_bmh(M, n_tiles);
+  const bool pair = ti::pair_serves(true, M, n_tiles, N, KS);
+  const int NT = ti::pair_tokens(true, M, n_tiles, KS, may_cut);
+  // 256 weight rows per CTA, which halve the bytes of the activations, where no k split follows from the fewer tiles: 34816 x 5120,
+  // a step of 8 decodes 782 us, on pairs 789
+  const int BMH = !pair && M <= 8 && ti::pair_many(M, n_tiles) ? 2 : 1;
   int rc = ti::cached_map(&p.map_w, w, KB, n_tiles, BMH == 2 ? -32 : 0);
   if (rc) return rc;
   rc = ti::cached_map(&p.map_xh, x, 2 * K, M, pair ? NT / 2 : BN);
@@ -253,7 +251,9 @@ int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M,
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (pair) {
-    ti::pair_apply(p, plan, n_tiles, NT, part, tile_count);
+    ti::pair_apply(p, ti::pair_plan(M, n_tiles, KS, NT, may_cut), n_tiles, NT, part, tile_count);
+    if (NT == 32) return ti::launch_pair<32, true>(p, st);
+    if (NT == 64) return ti::launch_pair<64, true>(p, st);
     return NT == 256 ? ti::launch_pair<256, true>(p, st) : ti::launch_pair<128, true>(p, st);
   }
   const int rows = ti::kBM * BMH;
@@ -261,8 +261,7 @@ int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M,
   const int S = ti::plan_split(p, KS, tiles_n * tiles_m, M, N, ldo, part, part_bytes, tile_count, n_count);
   dim3 grid(tiles_m, tiles_n, S);
   if (N <= 128 && M > 64 && BN == 32) return ti::launch_gemm<32, true, 1, ti::kGemmShortRingKb>(p, grid, st);   // two CTAs per SM
-  if (BMH == 2 && BN == 32) return ti::launch_gemm<32, true, 2>(p, grid, st);
-  if (BMH == 2 && BN == 64) return ti::launch_gemm<64, true, 2>(p, grid, st);
+  if (BMH == 2) return ti::launch_gemm<32, true, 2>(p, grid, st);
   if (BN == 32) return ti::launch_gemm<32, true>(p, grid, st);
   if (BN == 64) return ti::launch_gemm<64, true>(p, grid, st);
   return ti::launch_gemm<128, true>(p, grid, st);
