@@ -1,5 +1,5 @@
-"""The arg-max form of the top-k kernels (k = 1): ties, rows of -inf and of the lowest float, NaN, ragged vocabularies, and the
-static entry point; the oracle is the radix selection's order (float bits mapped to ascending integers, smallest id first)."""
+"""The arg-max form of the top-k kernels (k = 1): ties, rows of -inf and of the lowest float, NaN, ragged vocabularies, the merge of
+candidates in any order, and the static entry point; the oracle is the radix selection's order (float bits mapped to ascending integers, smallest id first)."""
 import ctypes
 
 import pytest
@@ -58,3 +58,28 @@ def test_top1(V):
         assert fn(d.data_ptr(), M, V, V, 1, 0, out_v.data_ptr(), out_i.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
         torch.cuda.synchronize()
         assert out_i[:, 0].cpu().tolist() == want
+
+
+@pytest.mark.parametrize("chunks", [2, 148, 600])
+def test_merge_of_candidates_in_any_order(chunks):
+    """Equal candidates whose ids do not ascend with their places (the arg-max epilogue of the vocabulary product deals columns
+    to CTAs by ticket): the smallest id wins, with its value, wherever it stands.  The last row has places without a candidate."""
+    from tileinfer_b200.ops import functional as F
+    F.L()
+    g = torch.Generator().manual_seed(chunks)
+    ids = torch.stack([torch.arange(chunks - 1, -1, -1), torch.randperm(chunks, generator=g), torch.randperm(chunks, generator=g),
+                       torch.arange(chunks).roll(1), torch.randperm(chunks, generator=g)]) * 3
+    val = torch.stack([torch.full((chunks,), 2.5), torch.randint(0, 2, (chunks,), generator=g).float(), torch.randn(chunks, generator=g),
+                       torch.full((chunks,), float("-inf")), torch.full((chunks,), torch.finfo(torch.float32).min)])
+    ids[4, torch.randperm(chunks, generator=g)[:chunks // 2]] = -1
+    want = [min((int(i) for i, v, k in zip(r, x, _key(x)) if i >= 0 and k == _key(x)[r >= 0].max()), default=-1) for r, x in zip(ids, val)]
+    M = len(val)
+    ws_v, ws_i = val.cuda(), ids.int().cuda()
+    out_v, out_i = torch.empty(M, 1, device="cuda"), torch.empty(M, 1, dtype=torch.int32, device="cuda")
+    p = F.TopkParams()
+    p.ws_val, p.ws_idx, p.out_val, p.out_idx = (t.data_ptr() for t in (ws_v, ws_i, out_v, out_i))
+    p.M, p.V, p.ld, p.k, p.chunks, p.chunk_size, p.vocab_start, p.tp = M, 3 * chunks, 0, 1, chunks, 0, 1000, 1
+    F.topk_merge(p)
+    torch.cuda.synchronize()
+    assert (out_i[:, 0].cpu() - 1000).tolist() == want
+    assert torch.equal(out_v[:, 0].cpu(), torch.stack([x[r >= 0].max() for r, x in zip(ids, val)]))

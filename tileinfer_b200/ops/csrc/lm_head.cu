@@ -155,24 +155,23 @@ TI_DEVICE void select_topk(float (&val)[EPT], int (&idx)[EPT], int k, float* out
   __syncthreads();
 }
 
-// The one best of a block (k = 1, greedy rows): largest key, then smallest position, of what each of the 256 threads found;
+// The one best of a block (k = 1, greedy rows): largest key, then smallest token id, of what each of the 256 threads found;
 // key 0 where there is no element at all.  Every thread gets the answer.
 struct Best {
   uint32_t key;
-  unsigned pos;
+  unsigned id;
 };
+TI_DEVICE bool better(const Best& a, const Best& b) { return a.key > b.key || (a.key == b.key && a.id < b.id); }
 TI_DEVICE Best block_best(Best b) {
   __shared__ Best warp_best[8];
   const uint32_t top = __reduce_max_sync(0xffffffffu, b.key);
-  const unsigned pos = __reduce_min_sync(0xffffffffu, b.key == top ? b.pos : 0xffffffffu);
-  if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = Best{top, pos};
+  const unsigned id = __reduce_min_sync(0xffffffffu, b.key == top ? b.id : 0xffffffffu);
+  if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = Best{top, id};
   __syncthreads();
   b = warp_best[0];
 #pragma unroll
-  for (int w = 1; w < 8; ++w) {
-    const Best o = warp_best[w];
-    if (o.key > b.key || (o.key == b.key && o.pos < b.pos)) b = o;
-  }
+  for (int w = 1; w < 8; ++w)
+    if (better(warp_best[w], b)) b = warp_best[w];
   return b;
 }
 
@@ -200,8 +199,8 @@ __global__ void __launch_bounds__(256) top1_stage1_kernel(const __grid_constant_
   }
   b = block_best(b);
   if (threadIdx.x == 0) {
-    p.ws_val[(size_t)m * p.chunks + c] = b.key ? row[b.pos] : -INFINITY;
-    p.ws_idx[(size_t)m * p.chunks + c] = b.key ? (int)b.pos : -1;
+    p.ws_val[(size_t)m * p.chunks + c] = b.key ? row[b.id] : -INFINITY;
+    p.ws_idx[(size_t)m * p.chunks + c] = b.key ? (int)b.id : -1;
   }
 }
 
@@ -236,16 +235,22 @@ __global__ void __launch_bounds__(256) topk_stage2_kernel(const __grid_constant_
   const int nc = p.chunks * p.k;
   const float* cv = p.ws_val + (size_t)m * nc;
   const int* ci = p.ws_idx + (size_t)m * nc;
-  if constexpr (ONE) {                             // candidates are in ascending order of their token ids
+  if constexpr (ONE) {
+    // candidates come in any order: those of the arg-max epilogue of the vocabulary product (one per CTA, columns dealt to the
+    // CTAs by ticket) do not ascend with their token ids, so equal ones are told apart by the id, not by the place
     Best b{0u, 0xffffffffu};
+    float v = 0.f;
     for (int i = threadIdx.x; i < nc; i += 256) {
-      const uint32_t key = ci[i] >= 0 ? float_key(cv[i]) : 0u;
-      if (key > b.key) b = Best{key, (unsigned)i};
+      const Best o{float_key(cv[i]), (unsigned)ci[i]};
+      if (ci[i] >= 0 && better(o, b)) {
+        b = o;
+        v = cv[i];
+      }
     }
-    b = block_best(b);
-    if (threadIdx.x == 0) {
-      fin_v[0] = b.key ? cv[b.pos] : -INFINITY;
-      fin_i[0] = b.key ? ci[b.pos] : -1;
+    const Best top = block_best(b);
+    if (top.key == 0u ? threadIdx.x == 0 : (b.key == top.key && b.id == top.id)) {
+      fin_v[0] = top.key ? v : -INFINITY;
+      fin_i[0] = (int)top.id;                      // no candidate: -1
     }
   } else {
     __shared__ TopkSmem sm;
