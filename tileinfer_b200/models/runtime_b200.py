@@ -165,6 +165,16 @@ class DeviceRuntime:
         dev = torch.from_numpy(buf).to(self.dev, non_blocking=True)
         return [None if a is None else dev[layout[i][0]:layout[i][0] + a.size].view(a.shape) for i, a in enumerate(arrays)]
 
+    @staticmethod
+    def _row_numbers(rows, n: int) -> np.ndarray:
+        """`rows` of a matrix of n rows as numbers from 0 to n - 1: negative ones count from the end, as in any indexing, others
+        raise here (index_select takes neither, and fails on the device)."""
+        r = np.asarray(rows.cpu() if isinstance(rows, torch.Tensor) else rows, dtype=np.int64)
+        r = np.where(r < 0, r + n, r)
+        if r.size and not 0 <= r.min() <= r.max() < n:
+            raise IndexError(f"rows {rows} of a step with {n}")
+        return r
+
     def _topk_rows(self, logits, n, k):
         """Per-rank top-k (+ fused candidate exchange); rows in chunks of the peer buffer capacity."""
         cap = self.peer.m_cap if self.peer is not None else n
@@ -217,6 +227,7 @@ class DeviceRuntime:
             h["qg"][:] = (qg_seq, qg_tok0, qg_ntok)
         x.inputs.copy_(torch.from_numpy(buf), non_blocking=True)
         rows = batch.out_rows if batch.out_rows is not None else [c - 1 for c in batch.cu_seqlens[1:]]
+        rows = self._row_numbers(rows, T)
         x.cu, x.tiles, rows = self._upload(batch.cu_seqlens, [[t[i] for t in tiles] for i in (1, 2, 3)] if tiles else None, rows)
         self._prepare_step(x, batch)
         cur = self._run_layers(x)
@@ -441,10 +452,10 @@ class DeviceRuntime:
         rows = batch.out_rows if batch.out_rows is not None else [e - 1 for e in batch.cu_seqlens[1:]]
         if self._graph_serves(batch):
             self._decode_graph_step(batch, 1, keep_logits=True)
-            logits = self._last_graph.logits
-            return logits[:len(rows)].clone() if rows == list(range(len(rows))) else logits[rows]
+            logits, rows = self._last_graph.logits, self._row_numbers(rows, batch.num_seqs)
+            return logits[:len(rows)].clone() if np.array_equal(rows, np.arange(len(rows))) else logits[rows.tolist()]
         hidden = self.forward(batch)
-        return self.logits(hidden) if rows else torch.empty(0, self.v_local, device=self.dev)
+        return self.logits(hidden) if len(rows) else torch.empty(0, self.v_local, device=self.dev)
 
     def _status_ptr(self) -> int:
         """Device word the kernels of this executor OR their error bits into."""
@@ -482,8 +493,9 @@ class DeviceRuntime:
                 return self._read_tokens(self._last_graph.samp, n)
         else:
             hidden = self.forward(batch)
-            if list(sample_rows) != list(range(hidden.shape[0])):
-                hidden = hidden.index_select(0, self._upload(sample_rows)[0])
+            rows = self._row_numbers(sample_rows, hidden.shape[0])
+            if not np.array_equal(rows, np.arange(hidden.shape[0])):
+                hidden = hidden.index_select(0, self._upload(rows)[0])
             lg = self.logits(hidden)
             if spec.get("edits"):
                 t0 = StepCtx()
