@@ -44,6 +44,7 @@ def test_rows_of_a_step(rows, kind):
 
 def test_rows_by_default_and_none():
     assert _Host().forward(_batch([3, 1, 2]))[:, 0].tolist() == [2, 3, 5]
+    assert _Host().forward(_batch([0, 0, 2, 1]))[:, 0].tolist() == [2, 2, 1, 2]
     assert _Host().step_logits(_batch([3, 1, 2], [])).shape == (0, 3)
 
 

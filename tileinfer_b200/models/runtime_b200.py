@@ -226,8 +226,9 @@ class DeviceRuntime:
         if nq:
             h["qg"][:] = (qg_seq, qg_tok0, qg_ntok)
         x.inputs.copy_(torch.from_numpy(buf), non_blocking=True)
-        rows = batch.out_rows if batch.out_rows is not None else [c - 1 for c in batch.cu_seqlens[1:]]
-        rows = self._row_numbers(rows, T)
+        rows = [c - 1 for c in batch.cu_seqlens[1:]] if batch.out_rows is None else batch.out_rows
+        if batch.out_rows is not None or rows[0] < 0:           # (a first sequence without tokens)
+            rows = self._row_numbers(rows, T)
         x.cu, x.tiles, rows = self._upload(batch.cu_seqlens, [[t[i] for t in tiles] for i in (1, 2, 3)] if tiles else None, rows)
         self._prepare_step(x, batch)
         cur = self._run_layers(x)
@@ -449,13 +450,15 @@ class DeviceRuntime:
     def step_logits(self, batch) -> torch.Tensor:
         """Runs the step the way generation does (captured graph for decode-only steps) and returns the fp32 logits
         of this rank's vocabulary shard at `batch.out_rows` (default: the last token of every sequence)."""
-        rows = batch.out_rows if batch.out_rows is not None else [e - 1 for e in batch.cu_seqlens[1:]]
+        n, rows = batch.num_seqs, batch.out_rows
         if self._graph_serves(batch):
             self._decode_graph_step(batch, 1, keep_logits=True)
-            logits, rows = self._last_graph.logits, self._row_numbers(rows, batch.num_seqs)
-            return logits[:len(rows)].clone() if np.array_equal(rows, np.arange(len(rows))) else logits[rows.tolist()]
+            logits = self._last_graph.logits
+            if rows is not None:
+                rows = self._row_numbers(rows, n).tolist()
+            return logits[:n].clone() if rows is None or rows == list(range(n)) else logits[rows]
         hidden = self.forward(batch)
-        return self.logits(hidden) if len(rows) else torch.empty(0, self.v_local, device=self.dev)
+        return self.logits(hidden) if rows is None or len(rows) else torch.empty(0, self.v_local, device=self.dev)
 
     def _status_ptr(self) -> int:
         """Device word the kernels of this executor OR their error bits into."""
@@ -493,9 +496,8 @@ class DeviceRuntime:
                 return self._read_tokens(self._last_graph.samp, n)
         else:
             hidden = self.forward(batch)
-            rows = self._row_numbers(sample_rows, hidden.shape[0])
-            if not np.array_equal(rows, np.arange(hidden.shape[0])):
-                hidden = hidden.index_select(0, self._upload(rows)[0])
+            if list(sample_rows) != list(range(hidden.shape[0])):
+                hidden = hidden.index_select(0, self._upload(self._row_numbers(sample_rows, hidden.shape[0]))[0])
             lg = self.logits(hidden)
             if spec.get("edits"):
                 t0 = StepCtx()
