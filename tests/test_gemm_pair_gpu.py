@@ -72,3 +72,20 @@ def test_pair_products_into_padded_rows():
     assert bool((buf[:, 16400:] == 7.0).all())
     ref = x.double() @ w.t()
     assert float((buf[:, :16400].double() - ref).norm() / ref.norm()) < 2.0 ** -8
+
+
+# Stages of k from one to more than the ring has (6 to 10 of them; 121 weight tiles, so that some pairs run one tile and some two):
+# the commits that a copying warp waits for before its CTA leaves are those of the last ring fill, whole or not, of one tile or two.
+@pytest.mark.parametrize("quantize", [True, False])
+@pytest.mark.parametrize("M", [20, 50, 100, 300])
+@pytest.mark.parametrize("stages", [1, 2, 3, 5, 6, 7, 9, 10, 11, 13])
+def test_last_ring_fill(stages, M, quantize):
+    F, W, x, w = _operands(M, 30976, stages * (128 if quantize else 64), quantize)
+    limbs = F.quant_rows(x) if quantize else None
+    F.status_ptr()
+    before = F._STATUS.clone()
+    run = lambda: F.gemm_w8a16(W, limbs) if quantize else F.gemm_bf16(W, x)  # noqa: E731
+    got, ref = [run() for _ in range(4)], x.double() @ w.t()
+    assert float((got[0].double() - ref).norm() / ref.norm()) < 2.0 ** -8          # stored as bf16: 2^-9 at most
+    assert all(torch.equal(got[0], o) for o in got[1:])
+    assert torch.equal(F._STATUS, before)                      # no wait ran out

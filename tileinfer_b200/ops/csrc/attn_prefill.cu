@@ -261,6 +261,21 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
     else umma_bf16(d, a, b, idesc, acc);
   };
 
+  // PAIR, copying threads after their last copy, number `issued` of a ring of `stages`: before a CTA leaves, the commits on its
+  // `empty` barriers that nobody waits for have to arrive (those of both CTAs come from the first one's MMAs), and after a wait
+  // that ran out the copies already issued have to land (the first CTA counts the bytes of both and holds the second at the
+  // closing cluster barrier).
+  auto settle = [&](bool ok, uint32_t full, uint32_t empty, int issued, int stages) {
+    if (!PAIR) return;
+    const int last = max(0, issued - stages);
+    for (int i = last; i < issued && ok; ++i) {
+      ok = !*abort_flag && mbar_wait(empty + 8 * (i % stages), (uint32_t)((i / stages) & 1), kAttnWaitNs, p.status);
+      if (!ok) *abort_flag = 1;
+    }
+    if (!ok && rank == 0)
+      for (int i = last; i < issued; ++i) mbar_wait(full + 8 * (i % stages), (uint32_t)((i / stages) & 1), kPairDrainNs, p.status);
+  };
+
   if (warp == 0 || warp == kAttnProducerV) {
     // ------------------------------------------------------------ TMA producers: warp 0 Q and K, warp 6 V
     // (one thread's wait / expect / copy sequence is slower than the tensor pipe consumes a tile, so K and V are
@@ -272,7 +287,8 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
         const uint32_t q_of = lead(q_full), k_of = lead(k_full);
 #pragma unroll
         for (int s = 0; s < G::kSlabs; ++s) load_2d(q_s + s * (128 * 128), &p.map_q, head * D + s * 64, tok0, q_of);
-        for (int j = 0; j < ntiles && !*abort_flag; ++j) {
+        int j = 0;
+        for (; j < ntiles && !*abort_flag; ++j) {
           int blk[G::kPages];
 #pragma unroll
           for (int g = 0; g < G::kPages; ++g) blk[g] = bt[min(page0 + j * 8 + (int)rank * G::kPages + g, npages - 1)];   // pages past the end repeat the last one (masked)
@@ -286,12 +302,15 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
             else tma_load_4d(dst, &p.map_k, 0, 0, 0, (blk[g] * p.hkv + kh) * 2, k_of + 8 * st);
           }
         }
+        settle(j == ntiles, k_full, k_empty, j, NS);
+        if (PAIR && *abort_flag && rank == 0) mbar_wait(q_full, 0, kPairDrainNs, p.status);
       } else {
         // PAIR: a stage is half a tile (four pages), so that the first half of the next tile can be fetched while P V works on
         // the second half of this one
         constexpr int HV = PAIR ? 2 : 1, PG = 8 / HV, NSV = PAIR ? 2 : NS;
         const uint32_t v_of = lead(v_full);
-        for (int i = 0; i < HV * ntiles && !*abort_flag; ++i) {
+        int i = 0;
+        for (; i < HV * ntiles && !*abort_flag; ++i) {
           int blk[PG];
 #pragma unroll
           for (int g = 0; g < PG; ++g) blk[g] = bt[min(page0 + i * PG + g, npages - 1)];
@@ -302,6 +321,7 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
           for (int g = 0; g < PG; ++g)
             load_2d(v_s + (st * PG + g) * G::kVPage, &p.map_v, 0, (blk[g] * p.hkv + kh) * DV + (int)rank * G::kVCols, v_of + 8 * st);
         }
+        settle(i == HV * ntiles, v_full, v_empty, i, NSV);
       }
     }
   } else if (warp == 1) {
@@ -544,10 +564,9 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(p_done + 8 * (j & 1)) : "memory");
       }
-      if (ok) {                                            // every P V has completed: they complete in order
-        ok = mbar_wait(p_empty + 8 * ((ntiles - 1) & 1), (uint32_t)(((ntiles - 1) >> 1) & 1), kAttnWaitNs, p.status);
-        ok = __all_sync(0xffffffffu, ok);
-      }
+      for (int j = max(0, ntiles - 2); j < ntiles; ++j)    // every P V has completed, and the commits of both P tiles have arrived
+        ok = ok && mbar_wait(p_empty + 8 * (j & 1), (uint32_t)((j >> 1) & 1), kAttnWaitNs, p.status);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) *abort_flag = 1;
       float* sm = s_max + (ntiles & 1) * 256;
       sm[half * 128 + r] = l;
@@ -695,7 +714,7 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
     tc_fence_before();
   }
   __syncthreads();
-  if (PAIR) cluster_sync_all();                            // neither CTA leaves while the other may use its memory
+  if (PAIR) cluster_sync_all();                            // neither CTA leaves before the copying and softmax warps of both are through
   if (warp == 1) {
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, 512);

@@ -146,6 +146,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) gem
           if (!BF16) tma_pair_2d(dst + kStageA + kPlane, &p.map_xl, kb * kBK * kKS, x.m * NT + row, bar);
         }
       }
+      // Before a CTA leaves, the commits on its `empty` barriers for the last ring fill have to arrive: nobody else waits for
+      // them, and those of both CTAs come from the first one's MMAs.  After a wait that ran out the copies already issued have
+      // to land; the first CTA counts the bytes of both and holds the second at the closing cluster barrier.
+      const int last = max(0, it - kStages);
+      for (int k = last; k < it && ok; ++k)
+        if ((k & 1) == first) ok = mbar_wait(empty0 + 8 * (k % kStages), (k / kStages) & 1, kGemmWaitNs, p.status);
+      if (!ok && rank == 0)
+        for (int k = last; k < it; ++k)
+          if ((k & 1) == first) mbar_wait(full0 + 8 * (k % kStages), (k / kStages) & 1, kPairDrainNs, p.status);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -302,7 +311,7 @@ for (int z0 = 0; z0 < p.slices; z0 += 4) {            // the loads of four slice
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();                                             // neither CTA leaves while the other may use its memory
+  cluster_sync_all();                                             // neither CTA leaves before the copying warps of both are through
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kCols);

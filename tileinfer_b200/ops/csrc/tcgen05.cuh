@@ -197,6 +197,7 @@ TI_DEVICE bool mbar_wait_cluster(uint32_t bar, uint32_t parity, unsigned long lo
     }
   }
 }
+constexpr unsigned long long kPairDrainNs = 1000000;        // limit for copies in flight to land after an error: they take microseconds
 // Tiled copies of a CTA pair: the destination is this CTA's shared memory, the bytes are counted on `bar`, which may be the
 // other CTA's.  No multicast.
 TI_DEVICE void tma_pair_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
