@@ -210,7 +210,7 @@ __global__ void __launch_bounds__((AttnPrefillGeom<D, DV, MODE, PAIR>::kThreads)
   const int ntok = p.qt_ntok[tile];
   if (ntok <= 0) return;                                   // padding tile (uniform over the cluster)
   if (PAIR && (smem_u32(smem_raw) & 1023) != 0) {
-    if (threadIdx.x == 0) atomicOr(p.status, kStatusBadArgument);
+    if (threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, kStatusBadArgument);
     return;
   }
   const int seq = p.qt_seq[tile], tok0 = p.qt_tok0[tile];
