@@ -557,8 +557,8 @@ def test_gemv_rowpar_handoff_to_next_product_emulated_ranks(tp, M):
 @pytest.mark.parametrize("staged", [False, True])
 @pytest.mark.parametrize("state_bf16", [False, True])
 def test_gdn_decode_many_sequences_staged(state_bf16, staged):
-    """64 single-token sequences x 6 heads, the two decode kernels for large batches: column-split blocks (a cluster
-    of four blocks per head and sequence, 32 state columns each), and blocks that walk several sequences with the state
+    """64 single-token sequences x 6 heads, the two decode kernels for large batches: column-split blocks (four
+    blocks per head and sequence, 32 state columns each), and blocks that walk several sequences with the state
     staged through shared memory (bulk copies, inputs fetched one sequence ahead).  Both must equal the tiled kernel."""
     F = _F()
     torch.manual_seed(1)

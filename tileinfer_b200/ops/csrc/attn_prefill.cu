@@ -24,14 +24,14 @@
 // capped by cap * tanh(score / cap); where |score / cap| is known to stay small (normalised queries and keys) the tanh is
 // its power series and the softmax needs no running maximum at all: exp2 of a bounded score neither overflows nor
 // vanishes, so the scores of a tile are read once, two threads can share a query row (eight softmax warps, half of the keys
-// of a tile each), and with shared memory for two P tiles the next one is written while P V of this one runs.  Every wait is bounded; on expiry the status word is set, all roles leave their loops
-// and TMEM is freed.  No load carries a cluster-multicast qualifier.
+// of a tile each), and with shared memory for two P tiles the next one is written while P V of this one runs.  Every wait on an mbarrier is bounded;
+// on expiry the status word is set, all roles leave their loops and TMEM is freed.  No load carries a cluster-multicast qualifier.
 //
 // PAIR: two heads of one KV head, as a cluster of two CTAs (cta_group::2).  A CTA alone pulls all of K and V through L2 for its
 // 128 query rows, 128 KB per tile of 128 keys at D = 256: as many cycles as the tensor pipe needs for the tile, from single
 // buffers.  A pair's products have M = 256: each CTA holds its own queries, half of the keys of a tile (N of Q K^T) and half of
-// the value columns (N of P V), so half the bytes cross L2 per query, and K and V fit twice.  The first CTA issues all MMAs;
-// `full` barriers are its own and count both CTAs' bytes and softmax threads, `empty` and S barriers are arrived on in both.
+// the value columns (N of P V), so half the bytes cross L2 per query, and K fits twice, V once as two halves that are refilled
+// one by one.  The first CTA issues all MMAs; `full` barriers are its own and count both CTAs' bytes and softmax threads, `empty` and S barriers are arrived on in both.
 #include "tensor_map.cuh"
 
 namespace ti {
@@ -39,7 +39,7 @@ namespace ti {
 struct AttnPrefillParams {
   alignas(64) CUtensorMap map_q;   // bf16 [T][hq*D], box {64, 128}, 128B swizzle
   alignas(64) CUtensorMap map_k;   // bf16 [blocks*hkv*2 groups][D/64 slabs][8 keys][64], box {64, 8, D/64, 2}, 128B swizzle
-  alignas(64) CUtensorMap map_v;   // bf16 [blocks*hkv*D][16], box {16, D}, 32B swizzle
+  alignas(64) CUtensorMap map_v;   // bf16 [blocks*hkv*DV][16], box {16, DV} (PAIR: {16, DV / 2}), 32B swizzle
   const int* block_tables;         // [S, max_blocks]
   const int* positions;            // [T]
   const int* qt_seq;               // [num_tiles] sequence of the query tile

@@ -580,8 +580,9 @@ static int launch_gemm(const GemmParams& p, dim3 grid, cudaStream_t st) {
 }
 
 // k split that fills the 148 SMs when there are few output tiles; sets kb_per_split.  KB counts stages of 128 bytes
-// of k; a slice has at least 16 of them (TI_GEMM_SPLIT_STAGES).  Measured at 64 tokens on N = 5120 (us): K = 6144
-// unsplit 28.8, three slices 22.2; K = 17408 unsplit 57.5, three slices 32.3.
+// of k; a slice has at least 16 of them (TI_GEMM_SPLIT_STAGES).  Unsplit -> split, us, bf16 (what this kernel serves with a k that
+// long): at 2 to 8 tokens 5120 x 17408 48 -> 33, 5120 x 6144 19.8 -> 15.5, 4096 x 4096 13.8 -> 10.7, 2048 x 2048 7.6 -> 8.0; a router
+// of 64 x 4096 at 2 / 64 / 512 tokens 12.2 -> 7.1, 13.4 -> 10.9, 16.9 -> 12.6, one of 16 x 2048 7.2 -> 7.0, 8.4 -> 10.2, 10.1 -> 12.0.
 static int plan_split(GemmParams& p, int KB, int tiles, int M, int N, int ldo, void* part, size_t part_bytes,
                       void* tile_count, int n_count) {
   int S = 1;

@@ -280,7 +280,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) gem
               va[u] = vb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
               if (pre && m0 + c0 + tk + 8 * u < p.M && ns + 8 <= p.N) rr[u] = gemm_resid_load(p, m0 + c0 + tk + 8 * u, ns);
             }
-for (int z0 = 0; z0 < p.slices; z0 += 4) {            // the loads of four slices are in flight together
+            for (int z0 = 0; z0 < p.slices; z0 += 4) {            // the loads of four slices are in flight together
               float4 a[2][4], c[2][4];
 #pragma unroll
               for (int z = 0; z < 4; ++z)
@@ -322,11 +322,14 @@ struct PairPlan {
   int whole, cut, slices, kb_per_split;
   float rounds;                      // rounds of whole tiles that the launch takes (cut tiles count as their longest slice)
 };
-// Cutting the tiles of the last round along k costs a round trip of partial results through L2, about as long as 40 stages,
-// so it has to save 66 stages (128 bytes of k) of that round.  N = 5120, us without / with: K = 17408 int8 (136 stages) at
-// 128 tokens 50 / 35, 512 tokens 88 / 74, 1060 tokens 136 / 130; bf16 (272 stages) 61 / 47, 100 / 91, 185 / 165.  K = 6144 int8
-// (48 stages) at 128 tokens 23.3 / 24.9, 1060 tokens 53 / 57: not cut.  Tiles of 32 and 64 tokens carry a quarter or half of
-// the partial results through L2 and are bound by the weights' arrival, which a cut shares among more SMs: 30 stages.
+// Cutting the tiles of the last round along k costs a round trip of partial results through L2: about as long as 40 stages (of
+// 128 bytes of k) of an int8 tile of 128 tokens, 50 of a bf16 one of 256, 64 of a bf16 one of 128, whose stages are shorter.  So it has
+// to save 66 stages of that round, where each of the three gains.  N = 5120, us uncut / cut: int8 at 128 tokens K = 6144 (saves 32)
+// 21.0 / 22.9, 8192 (42) 25.7 / 24.8, 17408 (90) 46.6 / 35.2, at 1060 tokens K = 6144 (24) 49 / 51, 17408 (68) 132 / 125; bf16 at 128
+// tokens K = 4096 (42) 19.5 / 21.8, 6144 (64) 25.5 / 25.1, 17408 (181) 57.9 / 44.1, at 1060 tokens K = 6144 (48) 63.6 / 64.8, 8192 (64)
+// 83.2 / 80.6.  Tiles of 32 and 64 tokens carry a quarter or half of the partial results through L2 and are bound by the weights'
+// arrival, which a cut shares among more SMs: 30 stages.  int8 5120 x 6144 (saves 32) at 32 / 64 tokens 14.4 / 13.8, 15.4 / 17.0, 4096 x
+// 8192 (48) 17.5 / 14.7, 18.7 / 18.2, 5120 x 17408 (90) 32.6 / 22.4, 33.9 / 27.0: tiles of 64 gain from about 40 on.
 static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
   PairPlan q;
   const int tiles = (n_tiles * 8 + 255) / 256 * ((M + NT - 1) / NT);
@@ -356,15 +359,20 @@ static int pair_tokens(bool bf16, int M, int n_tiles, int KS, bool may_cut) {
 static bool pair_many(int M, int n_tiles) { return (n_tiles * 8 + 255) / 256 * ((M + 127) / 128) >= 120; }
 // Which products the pairs take.  Not
 //   * short ones, unless they have many tiles: the launch of a pair and its first ring fill take about 4 us longer (8192 x 512 at 70
-//     tokens 11.1 us on one CTA per tile against 14.5, at 250 15.8 / 15.3, at 512 28.8 -> 16.8);
+//     tokens 11.1 us on one CTA per tile against 14.5, at 250 15.8 / 15.3, at 512 28.8 -> 16.8; with many tiles, 30976 x 320 at 8 / 64 /
+//     128 / 1024 tokens int8 6.3 -> 6.6, 11.0 -> 9.4, 19.7 -> 13.3, 115 -> 71, bf16 at 16 / 64 / 128 / 1024 6.9 -> 7.7, 10.9 -> 9.3, 18.2 -> 12.1,
+//     69 -> 51);
 //   * a single tile of weight rows (routers), which would leave half of each pair idle;
 //   * bf16 products of up to 8 tokens, where weights alone are streamed, twice as many bytes as in int8 (5120 x 17408 at 4 tokens 33.3
 //     us against 35.7, a step of 3 decodes 757 / 763; at 14 decodes 841 -> 827, at 32 934 -> 908).
 // One tile per CTA -> pairs, us, on N x K: 34816 x 5120 at 64 / 128 / 1060 / 4096 tokens int8 37.8 -> 34.0, 56 -> 39, 327 -> 239,
 // 1085 -> 810, bf16 61 -> 61, 70 -> 62, 379 -> 298, 1238 -> 917; 5120 x 17408 at 64 tokens int8 28.2 -> 24.9, bf16 43.2 -> 40.9;
 // 5120 x 6144 int8 18.9 -> 16.1, 30 -> 27, 95 -> 60, 366 -> 186; 2048 x 2048 at 64 / 128 / 1060 tokens int8 12.2 -> 9.6, 18 -> 13, 19 -> 15.
-// At 4 tokens an int8 product alone gains nothing (18.5 -> 17.7, 10.6 -> 11.3, 8.9 -> 9.8), a decode step does, since the next
-// product's weights are requested earlier: 2 decodes of the 27B layers 551 -> 515 us, 5 599 -> 557, 12 652 -> 591, 64 1038 -> 976.
+// At 4 tokens an int8 product alone gains nothing (18.5 -> 17.7, 10.6 -> 11.3, 8.9 -> 9.8), nor does a bf16 one at 12 to 24 (12288 x
+// 2048 12.3 -> 13.8, 4096 x 4096 11.8 -> 12.8); a decode step does, since the next product's weights are requested earlier: 2 decodes
+// of the 27B layers 551 -> 515 us, 5 599 -> 557, 12 652 -> 591, 64 1038 -> 976.  The other four families' steps of 2 to 64 decodes (widths 2048
+// and 4096) with this rule against one tile per CTA: int8 0.6 to 10.2 % faster, bf16 at 12 and more between 1.0 %
+// slower (one step, within what runs differ by) and 11.6 % faster.
 static bool pair_serves(bool bf16, int M, int n_tiles, int N, int KS) {
   return N > 128 && !(bf16 && M <= 8) && (KS >= 16 || M > 256 || pair_many(M, n_tiles));
 }

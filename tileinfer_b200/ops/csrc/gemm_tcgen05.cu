@@ -61,10 +61,10 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const __nv_bfloat16* __
 }
 
 // The same for rows of up to 512 * 5 * 8 = 20480 elements in ONE pass: every thread keeps its (up to five) 16-byte
-// chunks of the row in registers between the statistics and the quantisation, so the row is read once.  The block is
-// as small as the row allows (K / 40 threads, rounded up to warps: 128 threads at K = 5120), so that many rows are in
-// flight per SM: a row is a load -> reduce -> reduce -> store chain of a few microseconds, and 8192 rows of 512 threads
-// each pass through an SM only four at a time.
+// chunks of the row in registers between the statistics and the quantisation, so the row is read once.  With more than 148
+// rows the block is as small as the row allows (K / 40 threads, rounded up to warps: 128 threads at K = 5120), so that many rows
+// are in flight per SM: a row is a load -> reduce -> reduce -> store chain of a few microseconds, and 8192 rows of 512 threads
+// each pass through an SM only four at a time.  Fewer rows have an SM each and take a thread per chunk (ti_quant_rows).
 __global__ void __launch_bounds__(512) quant_rows_fast_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
                                                               const __nv_bfloat16* __restrict__ norm_w, float eps, int K,
                                                               int8_t* __restrict__ xh, uint8_t* __restrict__ xl,
