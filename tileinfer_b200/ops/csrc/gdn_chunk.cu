@@ -697,34 +697,38 @@ __global__ void __launch_bounds__(256) gdn_chunk_finish_kernel(const __grid_cons
 }
 
 // Conv history after the step (z = 0) and at the snapshot points (z = 1 + point): the raw inputs of the last three
-// tokens before that position.  Grid (S, hv, 1 + num_snap).  Snapshot points lie at least three tokens into the
-// step (they are block-aligned), so only the z = 0 blocks ever read the old history they also overwrite.
+// tokens before that position.  Grid (S, hv, 1 + num_snap).  A point in the first two tokens of the step (the rest of a prompt
+// that ends a block there) still reads the old history, which the z = 0 block overwrites: that block writes those points itself,
+// each thread those of its channels, ahead of the history.
 __global__ void __launch_bounds__(128) gdn_conv_tail_kernel(const __grid_constant__ GdnChunkParams p, int DK, int DV) {
   const int s = blockIdx.x, vh = blockIdx.y, z = blockIdx.z;
   const int NCH = 2 * DK + DV;
   const int kh = vh / (p.hv / p.hk);
   if (p.seq_ck[s] == p.seq_ck[s + 1]) return;
-  const int t0 = p.cu[s], t1 = p.cu[s + 1];
-  int n = t1 - t0;
+  const int t0 = p.cu[s], n = p.cu[s + 1] - t0;
   __nv_bfloat16* hist = p.conv_state + ((size_t)p.slots[s] * p.hv + vh) * 3 * NCH;
-  __nv_bfloat16* dst = hist;
-  if (z > 0) {
-    if (p.snap_rel == nullptr) return;
-    const int rel = p.snap_rel[s * p.num_snap + z - 1];
-    if (rel <= 0 || rel > n) return;
-    n = rel;
-    dst = p.snap_conv + ((size_t)p.snap_idx[s * p.num_snap + z - 1] * p.hv + vh) * 3 * NCH;
-  }
+  auto point = [&](int j) { return p.snap_rel[s * p.num_snap + j]; };
+  auto entry = [&](int j) { return p.snap_conv + ((size_t)p.snap_idx[s * p.num_snap + j] * p.hv + vh) * 3 * NCH; };
+  if (z > 0 && (point(z - 1) < 3 || point(z - 1) > n)) return;
   for (int c = threadIdx.x; c < NCH; c += blockDim.x) {
     const int col = c < DK ? kh * DK + c : (c < 2 * DK ? p.hk * DK + kh * DK + (c - DK) : 2 * p.hk * DK + vh * DV + (c - 2 * DK));
-    __nv_bfloat16 v[3];
+    auto write = [&](__nv_bfloat16* dst, int end) {           // the three inputs before token `end` of the step
+      __nv_bfloat16 v[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int ti = n - 3 + j;                               // token of the step (negative: older than the step)
-      v[j] = ti >= 0 ? p.proj[(size_t)(t0 + ti) * p.ld + col] : hist[(size_t)(3 + ti) * NCH + c];
+      for (int j = 0; j < 3; ++j) {
+        const int ti = end - 3 + j;                           // token of the step (negative: older than the step)
+        v[j] = ti >= 0 ? p.proj[(size_t)(t0 + ti) * p.ld + col] : hist[(size_t)(3 + ti) * NCH + c];
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dst[(size_t)j * NCH + c] = v[j];
+    };
+    if (z > 0) {
+      write(entry(z - 1), point(z - 1));
+      continue;
     }
-#pragma unroll
-    for (int j = 0; j < 3; ++j) dst[(size_t)j * NCH + c] = v[j];
+    for (int j = 0; p.snap_rel != nullptr && j < p.num_snap; ++j)
+      if (point(j) > 0 && point(j) < 3 && point(j) <= n) write(entry(j), point(j));
+    write(hist, n);
   }
 }
 
