@@ -1008,9 +1008,9 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
   }
   if (tid == 0) {
     __threadfence();
-    const int fin = atomicAdd(p0.sched + 1, 1);
-    if ((fin + 1) % ncta == 0) {
+    if (atomicAdd(p0.sched + 1, 1) + 1 == ncta) {
       for (int i = 0; i < kMaxChain * 16; ++i) p0.sched[8 + i] = 0;
+      p0.sched[1] = 0;
       p0.sched[2] = 0;
       __threadfence();
     }
