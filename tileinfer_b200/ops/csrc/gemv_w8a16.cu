@@ -220,6 +220,12 @@ TI_DEVICE void imma_s8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uin
       : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+TI_DEVICE void imma_s8u8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 TI_DEVICE void imma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -228,31 +234,36 @@ TI_DEVICE void imma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uin
 }
 
 // ---------------------------------------------------------------- activation staging
+// The threads that stage: all of the CTA, or (gemv_stream.cuh) its first kThreads.
+struct WholeCta {
+  static TI_DEVICE int threads() { return (int)blockDim.x; }
+  static TI_DEVICE void sync() { __syncthreads(); }
+};
 // Per-row statistics scratch: red[nwarps][16] then rowv[16] (rrms), rows[16] (limb scale 2^(e-14)).
-TI_DEVICE void block_row_reduce(float (&v)[16], int M, float* red, float* out, int tid, bool is_max) {
-  const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+template <class Group> TI_DEVICE void block_row_reduce(float (&v)[16], int M, float* red, float* out, int tid, bool is_max) {
+  const int warp = tid >> 5, lane = tid & 31, nwarps = Group::threads() >> 5;
   for (int m = 0; m < M; ++m) {
     const float r = is_max ? warp_max(v[m]) : warp_sum(v[m]);
     if (lane == 0) red[warp * 16 + m] = r;
   }
-  __syncthreads();
+  Group::sync();
   if (tid < M) {
     float a = is_max ? 0.f : 0.f;
     for (int w = 0; w < nwarps; ++w) a = is_max ? fmaxf(a, red[w * 16 + tid]) : a + red[w * 16 + tid];
     out[tid] = a;
   }
-  __syncthreads();
+  Group::sync();
 }
 
 // Stages the k-slice [k_lo, k_hi) of up to 16 rows as two int8 limb planes.  XNORM: the rows are first
 // RMS-normalised with (1+w) (statistics over the full row) and rounded to bf16.
-TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, uint8_t* xl, int stride, float* scratch) {
+template <class Group> TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, uint8_t* xl, int stride, float* scratch) {
   const int tid = threadIdx.x;
   float* red = scratch;            // [16 warps][16]
   float* rrms = scratch + 256;     // [16]
   float* amax = scratch + 272;     // [16]
   float* inv = scratch + 288;      // [16]  2^(e-14): value of one fixed-point unit
-  const int nthreads = blockDim.x;
+  const int nthreads = Group::threads();
   // ---- single-row fast path (batch-1 decode): the row lives in registers, read from memory once
   if (p.M == 1 && (k_hi - k_lo) <= 40 * nthreads && (p.xmode != XNORM || (k_lo == 0 && k_hi == p.K))) {
     const int warp = tid >> 5, lane = tid & 31, nwarps = nthreads >> 5;
@@ -282,7 +293,7 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
       }
       ss = warp_sum(ss);
       if (lane == 0) red[warp] = ss;
-      __syncthreads();
+      Group::sync();
       float tot = 0.f;
       for (int w = 0; w < nwarps; ++w) tot += red[w];
       const float rr = rsqrtf(tot / (float)p.K + p.eps);
@@ -306,7 +317,7 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
       for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[j][i]));
     mx = warp_max(mx);
     if (lane == 0) red[32 + warp] = mx;
-    __syncthreads();
+    Group::sync();
     float a = 0.f;
     for (int w = 0; w < nwarps; ++w) a = fmaxf(a, red[32 + w]);
     int e = (int)((__float_as_uint(a) >> 23) & 0xffu) - 127;
@@ -329,14 +340,14 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
       *reinterpret_cast<uint2*>(xh + o) = make_uint2(hw[0], hw[1]);
       *reinterpret_cast<uint2*>(xl + o) = make_uint2(lw[0], lw[1]);
     }
-    __syncthreads();
+    Group::sync();
     return;
   }
   float acc[16];
   if (p.xmode == XNORM) {
 #pragma unroll
     for (int m = 0; m < 16; ++m) acc[m] = 0.f;
-    for (int c = tid; c < (p.K >> 3); c += blockDim.x) {
+    for (int c = tid; c < (p.K >> 3); c += nthreads) {
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
         if (m >= p.M) break;
@@ -346,15 +357,15 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
         for (int i = 0; i < 4; ++i) acc[m] += bf16lo(w4[i]) * bf16lo(w4[i]) + bf16hi(w4[i]) * bf16hi(w4[i]);
       }
     }
-    block_row_reduce(acc, p.M, red, rrms, tid, false);
+    block_row_reduce<Group>(acc, p.M, red, rrms, tid, false);
     if (tid < p.M) rrms[tid] = rsqrtf(rrms[tid] / (float)p.K + p.eps);
-    __syncthreads();
+    Group::sync();
   }
   // pass A: row maxima over the slice
 #pragma unroll
   for (int m = 0; m < 16; ++m) acc[m] = 0.f;
   const int c_lo = k_lo >> 3, c_hi = k_hi >> 3;
-  for (int c = c_lo + tid; c < c_hi; c += blockDim.x) {
+  for (int c = c_lo + tid; c < c_hi; c += nthreads) {
     uint4 nw = make_uint4(0, 0, 0, 0);
     if (p.xmode == XNORM) nw = ldg_cached16(p.norm_w + c * 8);
     const uint32_t n4[4] = {nw.x, nw.y, nw.z, nw.w};
@@ -375,7 +386,7 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
       }
     }
   }
-  block_row_reduce(acc, p.M, red, amax, tid, true);
+  block_row_reduce<Group>(acc, p.M, red, amax, tid, true);
   if (tid < p.M) {
     const float a = amax[tid];
     int e = (int)((__float_as_uint(a) >> 23) & 0xffu) - 127;
@@ -384,9 +395,9 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
     amax[tid] = exp2f((float)(14 - e));          // quantisation scale
     inv[tid] = exp2f((float)(e - 14));
   }
-  __syncthreads();
+  Group::sync();
   // pass B: quantise and store the limb planes
-  for (int c = c_lo + tid; c < c_hi; c += blockDim.x) {
+  for (int c = c_lo + tid; c < c_hi; c += nthreads) {
     uint4 nw = make_uint4(0, 0, 0, 0);
     if (p.xmode == XNORM) nw = ldg_cached16(p.norm_w + c * 8);
     const uint32_t n4[4] = {nw.x, nw.y, nw.z, nw.w};
@@ -417,12 +428,12 @@ TI_DEVICE void stage_limbs(const GemvParams& p, int k_lo, int k_hi, int8_t* xh, 
       *reinterpret_cast<uint2*>(xl + o) = make_uint2(lw[0], lw[1]);
     }
   }
-  __syncthreads();
+  Group::sync();
 }
 
 // bf16-weight path: up to 16 rows into shared memory as bf16, RMS-normalised with (1+w) if the product wants that.
-TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride, float* scratch) {
-  const int tid = threadIdx.x, chunks = p.K >> 3, nthreads = blockDim.x;
+template <class Group> TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride, float* scratch) {
+  const int tid = threadIdx.x, chunks = p.K >> 3, nthreads = Group::threads();
   const bool norm = p.xmode == XNORM;
   float* red = scratch;
   float* rrms = scratch + 256;
@@ -447,7 +458,7 @@ TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride,
       }
       ss = warp_sum(ss);
       if (lane == 0) red[warp] = ss;
-      __syncthreads();
+      Group::sync();
       float tot = 0.f;
       for (int w = 0; w < nwarps; ++w) tot += red[w];
       rr = rsqrtf(tot / (float)p.K + p.eps);
@@ -467,7 +478,7 @@ TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride,
       }
       *reinterpret_cast<uint4*>(xs + c * 8) = o;
     }
-    __syncthreads();
+    Group::sync();
     return;
   }
   if (norm) {
@@ -484,9 +495,9 @@ TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride,
         for (int i = 0; i < 4; ++i) acc[m] += bf16lo(w4[i]) * bf16lo(w4[i]) + bf16hi(w4[i]) * bf16hi(w4[i]);
       }
     }
-    block_row_reduce(acc, p.M, red, rrms, tid, false);
+    block_row_reduce<Group>(acc, p.M, red, rrms, tid, false);
     if (tid < p.M) rrms[tid] = rsqrtf(rrms[tid] / (float)p.K + p.eps);
-    __syncthreads();
+    Group::sync();
   }
   for (int c = tid; c < chunks; c += nthreads) {
     const uint4 nw = norm ? ldg_cached16(p.norm_w + c * 8) : make_uint4(0, 0, 0, 0);
@@ -505,7 +516,7 @@ TI_DEVICE void stage_bf16(const GemvParams& p, __nv_bfloat16* xs, int xs_stride,
       *reinterpret_cast<uint4*>(xs + (size_t)m * xs_stride + c * 8) = o;
     }
   }
-  __syncthreads();
+  Group::sync();
 }
 
 // ---------------------------------------------------------------- work decomposition
@@ -834,8 +845,8 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
       if (stamp) p0.dbg[cta * 32 + 9 + 4 * op] = globaltimer_ns();
       lstride = limb_stride(p.K);
       xl = smem + (size_t)p.M * lstride;
-      if (WT == W_INT8) stage_limbs(p, 0, p.K, xh, xl, lstride, scratch);
-      else if (rows_staged(p.xmode, p.M, p.K)) stage_bf16(p, xs, p.K + 8, scratch);
+      if (WT == W_INT8) stage_limbs<WholeCta>(p, 0, p.K, xh, xl, lstride, scratch);
+      else if (rows_staged(p.xmode, p.M, p.K)) stage_bf16<WholeCta>(p, xs, p.K + 8, scratch);
       if (WT == W_INT8) {
         inv0 = g < p.M ? scratch[288 + g] : 0.f;
         inv1 = g + 8 < p.M ? scratch[288 + g + 8] : 0.f;
@@ -1105,6 +1116,8 @@ static int launch(const ChainParams& c, int ncta, cudaStream_t st, const ChainPa
 
 }  // namespace ti
 
+#include "gemv_stream.cuh"
+
 extern "C" {
 
 int ti_gemv_params_size() { return (int)sizeof(ti::GemvParams); }
@@ -1116,7 +1129,23 @@ int ti_gemv_chain(ti::ChainParams* c, int wt, int ncta, void* stream) {
   const int rc = ti::prepare(*c, wt);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  ti::StreamPlan q;
+  if (ti::stream_plan(*c, wt, q)) {
+    c->x_bytes = q.x_bytes;
+    if (q.rows == 1) return wt == ti::W_INT8 ? ti::launch_stream<ti::W_INT8, 1>(*c, q, ncta, st) : ti::launch_stream<ti::W_BF16, 1>(*c, q, ncta, st);
+    return wt == ti::W_INT8 ? ti::launch_stream<ti::W_INT8, 8>(*c, q, ncta, st) : ti::launch_stream<ti::W_BF16, 8>(*c, q, ncta, st);
+  }
   return wt == ti::W_INT8 ? ti::launch<ti::W_INT8>(*c, ncta, st, nullptr, 1) : ti::launch<ti::W_BF16>(*c, ncta, st, nullptr, 1);
+}
+
+// Where a CTA's part of a product lies (gemv_stream.cuh): first row tile, row tiles, first of a pair of left-over tiles or -1, the
+// pair's first and last k tile for this CTA, row tiles of the pair, slices.
+int ti_gemv_stream_part(int n_tiles, int KB, int skew, int cta, int ncta, int* out) {
+  const ti::StreamPart q = ti::stream_part(n_tiles, KB, ti::stream_slices(n_tiles, KB, ncta), skew, cta, ncta);
+  const ti::StreamUnit x = ti::stream_unit(q, n_tiles, KB, ncta, 0);
+  const int v[7] = {q.first, q.count, q.pair < 0 ? -1 : x.tile, q.kt0, q.kt1, x.two ? 2 : 1, q.slices};
+  for (int i = 0; i < 7; ++i) out[i] = v[i];
+  return 0;
 }
 
 // Size `c` exactly as ti_gemv_chain would (validation + x_bytes) without launching.

@@ -449,7 +449,7 @@ class GemvWorkspace:
     """Split-k partial buffer and per-tile arrival counters shared by all GEMV launches of a stream."""
 
     def __init__(self, device="cuda", max_units: int = 1 << 16, max_tiles: int = 1 << 16):
-        self.ws = torch.empty(max_units * 128, dtype=torch.float32, device=device)
+        self.ws = torch.zeros(max_units * 128, dtype=torch.float32, device=device)      # (zero: a tag no packet has)
         self.counters = torch.zeros(max_tiles, dtype=torch.int32, device=device)
         self.sched = torch.zeros(128, dtype=torch.int32, device=device)     # dynamic unit scheduling state
         self.max_units, self.max_tiles = max_units, max_tiles
@@ -477,8 +477,9 @@ def make_gemv_params(W: LinearW, x, out, M, *, xmode=XGLOBAL, epi=EPI_STORE, nor
     R, tps, stages = plan
     if ws is None:
         ws = default_workspace()
+    if ws.ws.numel() >= 1 << 18 and ws.counters.numel() >= NUM_SMS:      # (the parts gemv_stream.cuh uses: 1 MB, a counter per pair)
+        p.ws, p.counters = ptr(ws.ws), ptr(ws.counters)
     p.M, p.N, p.n_tiles, p.K, p.KB, p.S, p.kb_per_split = M, W.N, W.n_tiles, W.K, W.KB, 1, W.KB
-    p.ws = ptr(ws.ws)
     p.ldx = ldx if ldx is not None else (x.stride(0) if x.dim() > 1 else W.K)
     p.ldo = ldo if ldo is not None else (out.stride(0) if out.dim() > 1 else W.N)
     p.eps = eps

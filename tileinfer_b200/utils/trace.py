@@ -50,7 +50,7 @@ def nvtx_end():
 
 # kernel-name keywords -> category; first match wins (names of this package's kernels first, then ATen / NCCL)
 CATEGORIES = (
-    ("GEMV (W8A16 / bf16, fused norm / SwiGLU / all-reduce)", ("gemv_kernel",)),
+    ("GEMV (W8A16 / bf16, fused norm / SwiGLU / all-reduce)", ("gemv_",)),
     ("GEMM (tcgen05)", ("gemm_w8a16_kernel", "quant_rows")),
     ("Fused all-reduce (many rows)", ("ar_rows_kernel",)),
     ("Attention", ("attn_kernel", "attn_merge", "attn_prefill", "qkv_prep")),
