@@ -11,6 +11,7 @@ namespace ti {
 __global__ void embed_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                              __nv_bfloat16* __restrict__ out, int H, int vocab, unsigned* step) {
   const int m = blockIdx.x;
+  pdl_trigger();                                         // the first product's weights are requested meanwhile
   long long id = ids[m];
   if (id < 0 || id >= vocab) id = 0;
   const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)id * H);
@@ -31,7 +32,8 @@ TI_DEVICE float block_sum(float v, float* red) {
 }
 
 // y = rmsnorm(x + add?) * (one_plus ? 1 + w : w); optionally also writes the sum r = x + add.
-// One block per row; rows of any multiple of 8 elements.
+// One block per row; rows of any multiple of 8 elements.  A programmatic launch, like the products around it: without that the
+// next product's weights were requested only when this kernel had ended (3 us each, nine times in a step of bf16 weights).
 __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ add,
                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                __nv_bfloat16* __restrict__ r_out, int H, float eps, int one_plus) {
@@ -40,6 +42,8 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
   float* red = row + H;                                  // [32]
   const size_t base = (size_t)blockIdx.x * H;
   float ss = 0.f;
+  pdl_trigger();
+  pdl_wait();
   for (int c = threadIdx.x; c < H / 8; c += blockDim.x) {
     const uint4 v = *reinterpret_cast<const uint4*>(x + base + c * 8);
     uint32_t a4[4] = {v.x, v.y, v.z, v.w};
@@ -129,10 +133,9 @@ int ti_rmsnorm(const void* x, const void* add, const void* w, void* y, void* r_o
     attr = true;
   }
   const int threads = H >= 2048 ? 256 : 64;
-  ti::rmsnorm_kernel<<<M, threads, sm, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)add,
-                                                               (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-                                                               (__nv_bfloat16*)r_out, H, eps, one_plus);
-  return (int)cudaGetLastError();
+  const cudaError_t e = ti::launch_kernel(ti::rmsnorm_kernel, dim3(M), dim3(threads), sm, (cudaStream_t)stream, true, (const __nv_bfloat16*)x,
+                                          (const __nv_bfloat16*)add, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)r_out, H, eps, one_plus);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 int ti_act_mul(const void* a, const void* b, void* out, int M, int n, int lda, int ldb, int ldo, int mode,
