@@ -347,11 +347,16 @@ static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
 static bool pair_may_cut(const void* part, size_t part_bytes, const void* tile_count, int n_count) {
   return part != nullptr && tile_count != nullptr && part_bytes >= (size_t)kPairs * 256 * 256 * 4 && n_count >= kPairs;
 }
-// Tokens of a pair's tile.  Batched decode: as few as hold the batch.  bf16 products of many tokens: 128-token tiles cost 0.62 of
+// Tokens of a pair's tile.  Batched decode: as few as hold the batch.  A few hundred tokens of few weight tiles: 64, where that
+// gives more pairs work in the one round there is (and the round would not be cut along k instead): a tile of 64 takes about 0.7 of one
+// of 128.  us with tiles of 128 / 64, int8: 5120 x 6144 at 65 / 128 / 192 tokens 19.4 / 15.4, 21.4 / 16.3, 21.9 / 16.7, 2048 x 6144 at 128 / 512
+// 20.8 / 14.6, 21.3 / 16.9, 6176 x 2048 at 128 12.2 / 9.7; bf16: 5120 x 6144 at 128 24.7 / 22.8, 2048 x 6144 at 512 33.3 / 23.3.  bf16 products of many tokens: 128-token tiles cost 0.62 of
 // 256-token ones (34816 x 5120 at 4096 tokens: 1143 us against 917), but leave fewer pairs idle in the last round (5120 x 6144 at
 // 4096 tokens: 221 against 257).
 static int pair_tokens(bool bf16, int M, int n_tiles, int KS, bool may_cut) {
   if (M <= 64) return M <= 32 ? 32 : 64;
+  const int tn = (n_tiles * 8 + 255) / 256, t64 = tn * ((M + 63) / 64);
+  if (t64 <= kPairs && t64 > tn * ((M + 127) / 128) && pair_plan(M, n_tiles, KS, 128, may_cut).slices == 1) return 64;
   if (!bf16 || M <= 128) return 128;
   return 0.62f * pair_plan(M, n_tiles, KS, 128, may_cut).rounds < pair_plan(M, n_tiles, KS, 256, may_cut).rounds ? 128 : 256;
 }
