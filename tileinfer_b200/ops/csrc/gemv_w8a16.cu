@@ -1,4 +1,5 @@
-// Skinny W8A16 / bf16 matrix product for decode: y[M<=16, N] = x[M, K] * W[N, K]^T.
+// Skinny W8A16 / bf16 matrix product for decode: y[M<=16, N] = x[M, K] * W[N, K]^T.  Launches of up to 8 rows without packets between
+// ranks take the form of gemv_stream.cuh (stream_plan); this file has the other one and what both share.
 //
 // Replaces the reference's dequantize_gemv_kernel (kernels/splitk_gemv.py:131-201), which serves
 // M == 1 only with 64-bit weight loads, and its M > 1 fallback that re-materialises a bf16 copy of
