@@ -33,6 +33,7 @@ struct Consumers {
   static TI_DEVICE void sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads) : "memory"); }
 };
 TI_DEVICE void sync_with_epilogue() { asm volatile("bar.sync 2, %0;\n" ::"n"(kThreads + 32) : "memory"); }
+TI_DEVICE void tell_epilogue() { asm volatile("bar.arrive 2, %0;\n" ::"n"(kThreads + 32) : "memory"); }
 
 // A CTA's part of a product: a slice of a pair of left-over row tiles (or none), then row tiles first .. first + count.
 // Left-over tiles, one for some of the CTAs, lengthen a product of few row tiles per CTA (N = 5120: 640 tiles, 4.3 for each of 148
@@ -477,6 +478,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
       }
       if (dbg != nullptr && tid == 0) dbg[11 + 4 * op] = globaltimer_ns();
     }
+    __syncwarp();
+    tell_epilogue();                                         // nothing of the launch's state is read any more
   } else {
     // ------------------------------------------------------------ epilogue: lane -> weight row (lane & 15), half of the warps' sums
     typedef StreamSum<WT> Sum;
@@ -645,7 +648,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
         }
       }
     }
-    if (lane == 0) {                                         // the last CTA of the launch sets the counters back for the next one
+    // The last CTA of the launch sets the counters back for the next one, and the tag on.  The consumers read the tag: a CTA without a
+    // row tile in any product has nothing else in which its epilogue warp would wait for them.
+    __syncwarp();
+    sync_with_epilogue();
+    if (lane == 0) {
       __threadfence();
       if (atomicAdd(p0.sched + 1, 1) + 1 == ncta) {
         p0.sched[1] = 0;
