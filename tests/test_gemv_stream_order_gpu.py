@@ -57,3 +57,34 @@ def test_ctas_without_work(quant):
     from tileinfer_b200.ops import functional as F
     F.L()
     _agree(F, [(64, 128, F.EPI_ROWPAR), (256, 64, F.EPI_SWIGLU), (64, 128, F.EPI_ROWPAR), (136, 64, F.EPI_STORE)], 1, quant, 40)
+
+
+def test_a_long_kernel_before_the_launch():
+    """The launch starts early and fills its ring beside the kernel before it.  That one may take longer than the 2 s after which this
+    launch's waits give up (here: the packets of a second rank never come, which it notices after 2.3 s): the limit counts from its end."""
+    from tileinfer_b200.ops import functional as F
+    F.L()
+    N, K, ms = 1184 * 8, 4096, 2300                            # eight row tiles and 16 stages per CTA: more than the ring holds
+    g = torch.Generator(device="cuda").manual_seed(3)
+    W, W0 = (F.LinearW(torch.randn(n, k, generator=g, device="cuda") * k ** -0.5, True) for n, k in ((N, K), (64, 64)))
+    x, x0 = (torch.randn(1, k, generator=g, device="cuda").to(BF16) for k in (K, 64))
+    want = F.gemv(W, x, epi=F.EPI_F32)
+
+    class Comm:
+        tp, rank, m_cap, timeout_ns = 2, 0, 1, ms * 10 ** 6
+    boxes = [torch.zeros(2 * 2 * 32 * 16, dtype=torch.uint8, device="cuda") for _ in range(2)]       # this rank's packets, the other's
+    ctrl = torch.tensor([1, 0, 0, 0], dtype=torch.int32, device="cuda")
+    comm = Comm()
+    comm.ll_ptrs, comm.step_ptr, comm.status_ptr = [b.data_ptr() for b in boxes], ctrl.data_ptr(), ctrl.data_ptr() + 4
+    h, resid, out = torch.zeros(1, 64, dtype=BF16, device="cuda"), torch.zeros(1, 64, dtype=BF16, device="cuda"), torch.zeros(1, N, device="cuda")
+    ws = [F.GemvWorkspace(), F.GemvWorkspace()]
+    before = F.make_gemv_params(W0, x0, h, 1, epi=F.EPI_ROWPAR, resid=resid, ws=ws[0], comm=comm)
+    after = F.make_gemv_params(W, x, out, 1, epi=F.EPI_F32, ws=ws[1])
+    F.status_ptr()
+    status = F._STATUS.clone()
+    torch.cuda.synchronize()
+    F.gemv_launch(before, F.W_INT8)
+    F.gemv_launch(after, F.W_INT8)
+    torch.cuda.synchronize()
+    assert int(ctrl[1]) == 1                                   # the kernel before did wait that long
+    assert torch.equal(F._STATUS, status) and torch.equal(out, want)

@@ -355,6 +355,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
           const uint32_t step = (uint32_t)x.per * 512u;
           for (uint32_t left = (uint32_t)(x.kt1 - x.kt0) * 512u; left > 0;) {
             const uint32_t bytes = min(step, left), bar = full0 + 8 * s;
+            // The ring is full once.  From here on the copies wait for the consumers, who start when the kernel before has ended: its
+            // time is none of this launch's, whose limit is 2 s (between ranks it may itself wait that long for a peer).
+            if (issued == stages) pdl_wait();
             ok = stream_wait(empty0 + 8 * s, ph, p0.status);
             if (ok && issued >= flight) {
               ok = stream_wait(full0 + 8 * f, fph, p0.status);
