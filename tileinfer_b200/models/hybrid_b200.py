@@ -321,7 +321,7 @@ class _StepMixin:
             if limbs is None:
                 limbs = self._limbs[M, W.K] = F.Limbs(M, W.K, self.dev)
             F.quant_rows(xs, norm_w=norm_w, eps=self.cfg.rms_eps, out=limbs)
-            F.gemm_w8a16(W, limbs, out=out, epi=gepi, resid=r)
+            F.gemm_w8a16(W, limbs, out=out, epi=gepi, resid=r, status=self._status_ptr())
             self._launches += 2
             return
         if norm_w is not None:
@@ -330,7 +330,7 @@ class _StepMixin:
         elif xs.stride(0) != W.K:
             xs = xs.contiguous()
             self._launches += 1
-        F.gemm_bf16(W, xs, out=out, epi=gepi, resid=r)
+        F.gemm_bf16(W, xs, out=out, epi=gepi, resid=r, status=self._status_ptr())
         self._launches += 1
 
     def _gemv(self, W: LinearW, x, out, M, *, xmode, epi, norm_w=None, resid=None, ldo=None, out_idx=None):
@@ -361,7 +361,7 @@ class _StepMixin:
                 resid=None if resid is None else resid[m0:m0 + m], ws=self.ws, eps=self.cfg.rms_eps,
                 ldx=x.stride(0), ldo=out.stride(0) if ldo is None else ldo,
                 comm=self.peer if epi == EPI_ROWPAR else None, order=order, xll=xll,
-                out_idx=None if out_idx is None else out_idx[m0:m0 + m])
+                out_idx=None if out_idx is None else out_idx[m0:m0 + m], status=self._status_ptr())
             if M <= step and self.chain:
                 # dependent products are collected and launched together (up to four per launch)
                 if self._pending and (self._pending_wt != W.wt or len(self._pending) >= F.MAX_CHAIN):
@@ -384,12 +384,12 @@ class _StepMixin:
             limbs = F.Limbs(M, W.K, self.dev)
             F.ar_rows(self.peer, pend["parity"], M, W.K, pend["resid"], x, order=pend["order"], mode=F.AR_LIMBS,
                       norm_w=norm_w, limbs=limbs, eps=self.cfg.rms_eps, two_shot=self._two_shot(M))
-            F.gemm_w8a16(W, limbs, out=out[:M], epi=gepi, resid=r)
+            F.gemm_w8a16(W, limbs, out=out[:M], epi=gepi, resid=r, status=self._status_ptr())
         else:
             xn = torch.empty(M, W.K, dtype=BF16, device=self.dev)
             F.ar_rows(self.peer, pend["parity"], M, W.K, pend["resid"], x, order=pend["order"], mode=F.AR_BF16,
                       norm_w=norm_w, xn=xn, eps=self.cfg.rms_eps, two_shot=self._two_shot(M))
-            F.gemm_bf16(W, xn, out=out[:M], epi=gepi, resid=r)
+            F.gemm_bf16(W, xn, out=out[:M], epi=gepi, resid=r, status=self._status_ptr())
         self._launches += 2
 
     def _ar_flush(self):
@@ -464,7 +464,7 @@ class _StepMixin:
                 p.proj, p.conv_w, p.neg_a_exp, p.dt_bias, p.norm_w = ptr(x.proj), ptr(L.conv_w), ptr(L.neg_a_exp), ptr(L.dt_bias), ptr(L.norm_w)
                 p.state, p.conv_state = ptr(self.rec[ig]), ptr(self.conv[ig])
                 p.slots, p.cu, p.out = ptr(x.slots), ptr(x.cu), ptr(x.mix)
-                p.ld, p.hk, p.hv, p.eps = x.proj.stride(0), self.hk, self.hv, eps
+                p.ld, p.hk, p.hv, p.eps, p.status = x.proj.stride(0), self.hk, self.hv, eps, self._status_ptr()
                 if x.snap_rel is not None:
                     p.snap_rel, p.snap_idx, p.num_snap = ptr(x.snap_rel), ptr(x.snap_idx), x.num_snap
                     p.snap_state, p.snap_conv = ptr(x.snap_state[ig]), ptr(x.snap_conv[ig])
@@ -501,7 +501,7 @@ class _StepMixin:
                 q.positions, q.slot_mapping, q.q_out = ptr(x.positions), ptr(x.slot_mapping), ptr(x.qbuf)
                 q.kcache, q.vcache = ptr(self.kv[ia, 0]), ptr(self.kv[ia, 1])
                 q.ld, q.hq, q.hkv, q.rotary_dim = x.proj.stride(0), self.hq, self.hkv, c.rotary_dim
-                q.eps, q.log2_theta, q.num_blocks = eps, math.log2(c.rope_theta), self.num_blocks
+                q.eps, q.log2_theta, q.num_blocks, q.status = eps, math.log2(c.rope_theta), self.num_blocks, self._status_ptr()
                 self._flush()
                 F.qkv_prep(q, T, self.D)
                 a = AttnParams()
@@ -513,14 +513,14 @@ class _StepMixin:
                 a.out = ptr(mix)
                 a.hq, a.hkv, a.max_blocks, a.nsplit = self.hq, self.hkv, x.max_blocks, x.nsplit
                 a.ld, a.num_qg = x.proj.stride(0), x.num_qg
-                a.scale_log2e, a.num_blocks = self.D ** -0.5 * 1.4426950408889634, self.num_blocks
+                a.scale_log2e, a.num_blocks, a.status = self.D ** -0.5 * 1.4426950408889634, self.num_blocks, self._status_ptr()
                 F.attn_paged(a, self.D)
                 self._launches += 3 if x.num_qg else 1
                 if x.tiles is not None:
                     # sequences with many tokens in this step: 128-row query tiles on the tcgen05 tensor cores
                     F.attn_prefill(x.qbuf, self.kv[ia, 0], self.kv[ia, 1], self.num_blocks, x.block_tables, x.positions,
                                    x.tiles, x.proj, mix, hq=self.hq, hkv=self.hkv, D=self.D, max_blocks=x.max_blocks,
-                                   ld=x.proj.stride(0))
+                                   ld=x.proj.stride(0), status=self._status_ptr())
                     self._launches += 1
                 self._rowpar(L.o, mix, cur, nxt, T)
                 ia += 1

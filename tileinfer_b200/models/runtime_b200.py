@@ -414,7 +414,7 @@ class DeviceRuntime:
         t.par.copy_(t.h_par, non_blocking=True)
 
     def _read_tokens(self, t, n) -> list:
-        """The step's only device -> host copy: n token ids and the communicator's status word."""
+        """The step's only device -> host copy: n token ids and the executor's status word."""
         t.h_tok.copy_(t.tok, non_blocking=True)
         torch.cuda.current_stream().synchronize()
         self.check_status(int(t.h_tok[t.tok.shape[0] - 1]))

@@ -6,7 +6,7 @@
 // 1151-1169: torch.topk / softmax / sort / cumsum / multinomial with an `.item()` synchronisation per sequence and a
 // broadcast of the chosen ids from rank 0).  Here both kernels sit inside the CUDA-graph decode step: a request with
 // a penalty, a bias or a grammar stays on the graph path, and the only device -> host traffic of a step is the chosen
-// token id per row plus the communicator's status word, in one small copy.
+// token id per row plus the executor's status word, in one small copy.
 //
 // Every rank runs the same deterministic kernel on the same candidates (already exchanged by the top-k kernel) with
 // the same uniform number drawn by the host from a generator all ranks seed alike, so all ranks pick the same token

@@ -467,7 +467,8 @@ def default_workspace():
 
 def make_gemv_params(W: LinearW, x, out, M, *, xmode=XGLOBAL, epi=EPI_STORE, norm_w=None, resid=None, ws=None,
                      eps=1e-6, ldx=None, ldo=None, comm=None, order=0, ncta=NUM_SMS, team=None, xll=False,
-                     out_idx=None) -> GemvParams:
+                     out_idx=None, status=0) -> GemvParams:
+    """status: device word for the error bits (default: the process-wide one; a communicator's products use its own)."""
     p = GemvParams()
     p.w, p.scale, p.x, p.norm_w = ptr(W.tiles), ptr(W.scale), ptr(x), ptr(norm_w)
     p.out, p.resid, p.out_idx = ptr(out), ptr(resid), ptr(out_idx)
@@ -490,7 +491,7 @@ def make_gemv_params(W: LinearW, x, out, M, *, xmode=XGLOBAL, epi=EPI_STORE, nor
     if ws is None:
         ws = default_workspace()
     p.sched = ptr(ws.sched)
-    p.status = status_ptr()
+    p.status = status or status_ptr()
     p.tp, p.rank, p.order, p.m_cap = 1, 0, order, 0
     if comm is not None and comm.tp > 1:
         p.tp, p.rank, p.m_cap = comm.tp, comm.rank, comm.m_cap
@@ -664,7 +665,7 @@ def attn_paged(p: AttnParams, D: int, DV: int = None):
 
 def attn_prefill(q, kcache, vcache, num_blocks, block_tables, positions, tiles, gate_src, out, *, hq, hkv, D,
                  max_blocks, ld, DV=None, scale=None, softcap=0.0, qk_max=0.0, window=0, slopes=None, head_gate=None, gcol=0, out_scale=1.0,
-                 gate_col=0, gate_stride=0):
+                 gate_col=0, gate_stride=0, status=0):
     """Causal GQA attention of prefill query tiles on the tcgen05 tensor cores (ops/csrc/attn_prefill.cu).
     `tiles`: int32 [3, n] = (sequence, first flat token, tokens <= 128) per tile, longest KV first.  DV: size of a value
     head (default D); softcap: scores become softcap * tanh(scale q.k / softcap); qk_max: a bound of |q.k| where there is
@@ -677,7 +678,7 @@ def attn_prefill(q, kcache, vcache, num_blocks, block_tables, positions, tiles, 
                               ptr(tiles[0]), ptr(tiles[1]), ptr(tiles[2]), n, ptr(gate_src), ptr(out), hq, hkv,
                               max_blocks, ld, scale, D, D if DV is None else DV, softcap, qk_max, window, ptr(slopes), ptr(head_gate),
                               0 if head_gate is None else head_gate.stride(0), gcol, out.stride(0) if out.dim() == 2 else 0, out_scale, gate_col, gate_stride,
-                              status_ptr(), stream()),
+                              status or status_ptr(), stream()),
           "ti_attn_prefill")
 
 
@@ -761,7 +762,7 @@ def quant_rows(x: torch.Tensor, norm_w=None, eps: float = 1e-6, out: Limbs = Non
     return out
 
 
-def gemm_w8a16(W: "LinearW", limbs: Limbs, *, out=None, epi=GEPI_STORE, resid=None, ex=None) -> torch.Tensor:
+def gemm_w8a16(W: "LinearW", limbs: Limbs, *, out=None, epi=GEPI_STORE, resid=None, ex=None, status=0) -> torch.Tensor:
     """y = x W^T on the tcgen05 tensor cores for int8-tiled W and the limb planes of x (any M)."""
     assert W.wt == W_INT8 and limbs.K == W.K
     M = limbs.M
@@ -769,12 +770,12 @@ def gemm_w8a16(W: "LinearW", limbs: Limbs, *, out=None, epi=GEPI_STORE, resid=No
         out = torch.empty(M, W.N // 2 if epi == GEPI_SWIGLU else W.N, dtype=torch.bfloat16, device=limbs.hi.device)
     part, count = _gemm_workspace(limbs.hi.device)
     check(_l.lib().ti_gemm_w8a16(ptr(W.tiles), ptr(W.scale), W.n_tiles, W.N, W.K, ptr(limbs.hi), ptr(limbs.lo),
-                            ptr(limbs.scale), M, ptr(resid), ptr(out), out.stride(0), epi, status_ptr(), ptr(part),
+                            ptr(limbs.scale), M, ptr(resid), ptr(out), out.stride(0), epi, status or status_ptr(), ptr(part),
                             part.numel() * 4, ptr(count), count.numel(), _ref(ex), stream()), "ti_gemm_w8a16")
     return out
 
 
-def gemm_bf16(W: "LinearW", x: torch.Tensor, *, out=None, epi=GEPI_STORE, resid=None, ex=None) -> torch.Tensor:
+def gemm_bf16(W: "LinearW", x: torch.Tensor, *, out=None, epi=GEPI_STORE, resid=None, ex=None, status=0) -> torch.Tensor:
     """y = x W^T on the tcgen05 tensor cores (kind::f16) for bf16-tiled W and bf16 x [M, K] with contiguous rows.
     epi GEPI_F32 stores fp32 (logits)."""
     assert W.wt == W_BF16 and x.shape[1] == W.K and x.stride(1) == 1 and x.stride(0) == W.K and x.dtype == torch.bfloat16
@@ -784,7 +785,7 @@ def gemm_bf16(W: "LinearW", x: torch.Tensor, *, out=None, epi=GEPI_STORE, resid=
         out = torch.empty(M, cols, dtype=torch.float32 if epi == GEPI_F32 else torch.bfloat16, device=x.device)
     part, count = _gemm_workspace(x.device)
     check(_l.lib().ti_gemm_bf16(ptr(W.tiles), W.n_tiles, W.N, W.K, ptr(x), M, ptr(resid), ptr(out), out.stride(0), epi,
-                           status_ptr(), ptr(part), part.numel() * 4, ptr(count), count.numel(), _ref(ex), stream()), "ti_gemm_bf16")
+                           status or status_ptr(), ptr(part), part.numel() * 4, ptr(count), count.numel(), _ref(ex), stream()), "ti_gemm_bf16")
     return out
 
 
