@@ -107,3 +107,18 @@ def test_argmax(M):
     best = val.argmax(1)
     assert torch.equal(val.amax(1), logits.amax(1))
     assert torch.equal(idx.gather(1, best[:, None])[:, 0].long(), logits.argmax(1))
+
+
+@pytest.mark.parametrize("N", [64, 4744])
+def test_sums_of_a_long_row_fit_in_32_bits(N):
+    """K beyond 65536: low limbs of 255 beside weights of 127 add up to more than 2^31.  Every weight is 1, one activation (64) sets the
+    row's unit to 2^-8, all others are 255 units."""
+    F = _F()
+    K = 72000
+    W = F.LinearW(torch.ones(N, K, device="cuda"), True)
+    x = torch.full((1, K), 255 / 256, dtype=BF16, device="cuda")
+    x[0, 7] = 64.0
+    y = F.gemv(W, x, epi=F.EPI_F32).double()
+    want = x.double().sum() * 127 * W.scale[:N].double()
+    # exact integer sums, their two parts added in fp32 and scaled: a few roundings of 2^-24
+    assert not bool(((y[0] - want).abs() > 2.0 ** -21 * want).any())

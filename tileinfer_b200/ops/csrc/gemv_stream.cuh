@@ -676,7 +676,7 @@ static bool stream_plan(const ChainParams& c, int wt, StreamPlan& q) {
   int m = 0;
   for (int i = 0; i < c.n_ops; ++i) {
     const GemvParams& p = c.op[i];
-    if (p.tp > 1 || p.xll || p.M > kStreamMaxRows) return false;
+    if (p.tp > 1 || p.xll || p.M > kStreamMaxRows || (wt == W_INT8 && p.K > kMaxIntK)) return false;
     const size_t x = wt == W_INT8 ? (size_t)2 * p.M * limb_stride(p.K) : (size_t)p.M * (p.K + 8) * 2;
     q.x_bytes = std::max(q.x_bytes, (int)((x + 2048 + 127) / 128 * 128));
     q.slot_bytes = std::max(q.slot_bytes, stream_slot_bytes(wt, p.M));

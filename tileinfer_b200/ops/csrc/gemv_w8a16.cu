@@ -115,6 +115,7 @@ constexpr int kLook = 1;                   // entries a warp queues ahead of its
                                            // while it is still idle or busy elsewhere, and the product then ends on the few
                                            // warps that hold three or four units each
 constexpr int kMaxR = 4;                   // row tiles per unit
+constexpr int kMaxIntK = 65536;            // up to this K the largest sum of low limbs, 255 x 128 x K, is below 2^31
 constexpr int kTeamBytes = 2 * kWarps * 32 * 16;   // team-mode exchange buffer
 
 // Operands of the epilogue that do not depend on the product: fetched when a warp STARTS a row tile, so that
@@ -943,7 +944,7 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
       if (WT == W_INT8) {
 #pragma unroll
         for (int b = 0; b < 4; ++b)
-          acc[b] = ((float)(ah[0][b] + ah[1][b]) * 256.f + (float)(al[0][b] + al[1][b])) * (b < 2 ? inv0 : inv1);
+          acc[b] = ((float)(ah[0][b] + ah[1][b]) * 256.f + (p.K > kMaxIntK ? (float)((long long)al[0][b] + al[1][b]) : (float)(al[0][b] + al[1][b]))) * (b < 2 ? inv0 : inv1);
       }
       if (p.T > 1) {
         // partial sums of the team meet in shared memory (two alternating slots: the barrier of exchange n+1
