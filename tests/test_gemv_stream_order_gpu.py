@@ -19,7 +19,7 @@ def _chain(F, shapes, M, quant, seed=1):
         g = torch.Generator(device="cuda").manual_seed(seed)
         x = torch.randn(M, shapes[0][1], generator=g, device="cuda").to(BF16)
         hidden = [torch.randn(M, shapes[0][0], generator=g, device="cuda").to(BF16) for _ in range(2)]
-        cur, ps, outs = 0, [], []
+        cur, ps, outs, first = 0, [], [], x                    # (the parameters hold addresses: the input has to outlive the launch)
         for (n, k, epi), W, nw in zip(shapes, Ws, nws):
             if epi == F.EPI_ROWPAR:
                 out = hidden[1 - cur]
@@ -35,6 +35,7 @@ def _chain(F, shapes, M, quant, seed=1):
         else:
             for p in ps:
                 F.gemv_launch(p, Ws[0].wt)
+        del first
         return outs
     return run, ws
 
