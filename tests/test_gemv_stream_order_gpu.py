@@ -89,3 +89,29 @@ def test_a_long_kernel_before_the_launch():
     torch.cuda.synchronize()
     assert int(ctrl[1]) == 1                                   # the kernel before did wait that long
     assert torch.equal(F._STATUS, status) and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("M", [2, 8])
+def test_several_rows_behind_a_grid_barrier(M):
+    """bf16 rows that do not fit in 48 KB without a norm: the products of a chain are separated by grid barriers."""
+    from tileinfer_b200.ops import functional as F
+    F.L()
+    H = 24576 // M
+    g = torch.Generator(device="cuda").manual_seed(M)
+    Ws = [F.LinearW(torch.randn(H, H, generator=g, device="cuda") * H ** -0.5, False) for _ in range(3)]
+    ws = F.GemvWorkspace()
+    for seed in range(10):
+        x = torch.randn(M, H, generator=g, device="cuda").to(BF16)
+
+        def run(chained):
+            a, b = torch.zeros_like(x), torch.zeros_like(x)
+            ps = [F.make_gemv_params(Ws[0], x, a, M, ws=ws), F.make_gemv_params(Ws[1], a, b, M, ws=ws),
+                  F.make_gemv_params(Ws[2], b, a, M, epi=F.EPI_ROWPAR, resid=x, ws=ws)]
+            if chained:
+                F.gemv_chain_launch(ps, F.W_BF16)
+            else:
+                for p in ps:
+                    F.gemv_launch(p, F.W_BF16)
+            return a, b
+        assert all(torch.equal(u, v) for u, v in zip(run(False), run(True))), seed
+    assert int(ws.sched[:3].abs().sum()) == 0 and int(ws.counters.abs().sum()) == 0

@@ -1,6 +1,7 @@
-// The products of a decode step with up to 8 activation rows on one GPU: weights streamed through ONE ring per CTA.
+// The products of a decode step of one activation row on one GPU, and some bf16 ones of up to 8 rows (stream_rows): weights streamed
+// through ONE ring per CTA.
 //
-// The other form (gemv_body, kept for packets between ranks and for 9 to 16 rows) gives every warp units of its own, a private
+// The other form (gemv_body, for packets between ranks and for several rows) gives every warp units of its own, a private
 // ring and a lane that schedules and copies.  Its launch of a 27B layer's four products (383 MB, 58.5 us at the measured copy
 // rate) took 87.5 us, and as long with weights that stay in L2: 6 shared-memory loads and 8 MMAs per KB of weights, a lane's copy
 // and scheduling work in between, warps that end a product up to 15 us apart, and rings (128 KB) that are full long before the
@@ -670,8 +671,20 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
 }
 
 struct StreamPlan { int x_bytes, stages, slots, slot_bytes, rows; };
-// Whether a launch takes this form: one GPU's products of up to 8 rows, whose staged rows leave room for 4 stages.
-static bool stream_plan(const ChainParams& c, int wt, StreamPlan& q) {
+// Whether a product of several rows, or of one row longer than registers hold, takes this form: where gemv_body reads bf16 rows from
+// global memory anew for every tile (us, gemv_body / here: 16480 x 5120 at 6 / 8 rows 94.7 / 40.1, 93.7 / 47.1, 5120 x 6144 at 4 / 8 32.0 / 19.6, 31.6 /
+// 27.8, 8192 x 32768 at one 178 / 82), and for one row (8192 x 32768 int8 60.7 / 52.4, 3552 x 20544 22.8 / 22.2, a chain with K = 21504 107.8 / 99.5).
+// Other products of several rows do not: a stage of weights costs more here with every row (int8 16480 x 5120 at 2 / 4 / 8 rows 23.0 / 27.9, 25.1 /
+// 37.1, 31.1 / 56.7; bf16 32768 x 2048 at 4 / 8 29.5 / 31.3, 30.6 / 41.6).  Nor do those with few tiles per CTA, whose k the teams of gemv_body cut
+// in 16 (one int8 row 256 x 32768 16.8 / 20.2, 2048 x 32768 22.9 / 25.1, 2368 x 32768 24.8 / 23.4; 256 x 8192 eight bf16 rows 10.3 / 12.7).  A decode step of several rows takes the tensor-core
+// products.  Small products of several rows would gain (2048 x 2048 at 2 rows 10.1 / 7.9), but a chain would then not have the bits of its products
+// launched one by one.
+static bool stream_rows(const GemvParams& p, int wt, int ncta) {
+  if (wt == W_BF16 && !rows_staged(p.xmode, p.M, p.K)) return p.n_tiles > ncta;
+  return p.M == 1 && p.n_tiles >= 2 * ncta;
+}
+// Whether a launch takes this form: one GPU's products of up to 8 rows, whose staged rows leave room for 4 stages, if it is the faster one.
+static bool stream_plan(const ChainParams& c, int wt, int ncta, StreamPlan& q) {
   q.x_bytes = q.slot_bytes = 0;
   int m = 0;
   for (int i = 0; i < c.n_ops; ++i) {
@@ -683,6 +696,8 @@ static bool stream_plan(const ChainParams& c, int wt, StreamPlan& q) {
     m = std::max(m, p.K <= 40 * kThreads ? p.M : kStreamMaxRows);
   }
   q.rows = m;
+  for (int i = 0; m > 1 && i < c.n_ops; ++i)
+    if (!stream_rows(c.op[i], wt, ncta)) return false;
   q.slots = m <= 2 ? kStreamMaxSlots : 2;
   const int room = 227 * 1024 - 1024 - q.x_bytes - q.slots * q.slot_bytes;       // (1 KB static: barriers, parts)
   q.stages = std::min(kStreamMaxStages, room / kStreamStage);

@@ -1,5 +1,5 @@
-// Skinny W8A16 / bf16 matrix product for decode: y[M<=16, N] = x[M, K] * W[N, K]^T.  Launches of up to 8 rows without packets between
-// ranks take the form of gemv_stream.cuh (stream_plan); this file has the other one and what both share.
+// Skinny W8A16 / bf16 matrix product for decode: y[M<=16, N] = x[M, K] * W[N, K]^T.  Launches of one row without packets between ranks,
+// and some of bf16 weights of 2 to 8 rows, take the form of gemv_stream.cuh (stream_plan); this file has the other one and what both share.
 //
 // Replaces the reference's dequantize_gemv_kernel (kernels/splitk_gemv.py:131-201), which serves
 // M == 1 only with 64-bit weight loads, and its M > 1 fallback that re-materialises a bf16 copy of
@@ -1132,7 +1132,7 @@ int ti_gemv_chain(ti::ChainParams* c, int wt, int ncta, void* stream) {
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   ti::StreamPlan q;
-  if (ti::stream_plan(*c, wt, q)) {
+  if (ti::stream_plan(*c, wt, ncta, q)) {
     c->x_bytes = q.x_bytes;
     if (q.rows == 1) return wt == ti::W_INT8 ? ti::launch_stream<ti::W_INT8, 1>(*c, q, ncta, st) : ti::launch_stream<ti::W_BF16, 1>(*c, q, ncta, st);
     return wt == ti::W_INT8 ? ti::launch_stream<ti::W_INT8, 8>(*c, q, ncta, st) : ti::launch_stream<ti::W_BF16, 8>(*c, q, ncta, st);
@@ -1150,7 +1150,18 @@ int ti_gemv_stream_part(int n_tiles, int KB, int skew, int cta, int ncta, int* o
   return 0;
 }
 
-// Size `c` exactly as ti_gemv_chain would (validation + x_bytes) without launching.
+// Which form a launch of ti_gemv_chain takes: out = stages of its ring, the rows its kernel is built for (1, 8), bytes of staged rows
+// (gemv_stream.cuh), or zeros (the form of this file).
+int ti_gemv_stream_plan(const ti::ChainParams* c, int wt, int ncta, int* out) {
+  ti::StreamPlan q;
+  const bool yes = ti::stream_plan(*c, wt, ncta, q);
+  out[0] = yes ? q.stages : 0;
+  out[1] = !yes ? 0 : q.rows == 1 ? 1 : ti::kStreamMaxRows;
+  out[2] = yes ? q.x_bytes : 0;
+  return 0;
+}
+
+// Size `c` as the form of this file would (validation + x_bytes) without launching.
 int ti_gemv_chain_prepare(ti::ChainParams* c, int wt, int ncta) { return ti::prepare(*c, wt); }
 
 // One cooperative launch that runs `nranks` emulated ranks (prepared chain blocks in device memory at

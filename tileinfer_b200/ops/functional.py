@@ -398,7 +398,7 @@ TEAM_BYTES = 2 * GEMV_WARPS * 32 * 16      # exchange buffer of team mode (must 
 def plan_team(n_tiles: int, KB: int, R: int, team: int | None = None, ncta: int = NUM_SMS) -> int:
     """Team size T for a product: how many adjacent warps of a CTA share one unit, each streaming a slice of k.
     A product with fewer units than warps would leave warps (and the bytes they keep in flight) idle.
-    `team` (or TI_GEMV_T) forces a size.  Launches of up to 8 rows on one GPU (gemv_stream.cuh) have no teams.
+    `team` (or TI_GEMV_T) forces a size.  Launches of one row on one GPU (gemv_stream.cuh) have no teams.
 
     Cost model (in 512-byte tiles a warp streams one after the other): a CTA holds GEMV_WARPS // T whole teams,
     the units are dealt to the teams in waves, a unit costs ceil(KB / T) tiles per warp plus a fixed part (team

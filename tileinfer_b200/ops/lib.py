@@ -89,6 +89,7 @@ class _Sigs:
     ti_gemv_chain = (_I, [ctypes.POINTER(ChainParams), _I, _I, _P], "hybrid")
     ti_gemv_chain_prepare = (_I, [ctypes.POINTER(ChainParams), _I, _I], "hybrid")
     ti_gemv_ranks = (_I, [ctypes.POINTER(ChainParams), _P, _I, _I, _P], "hybrid")
+    ti_gemv_stream_plan = (_I, [ctypes.POINTER(ChainParams), _I, _I, ctypes.POINTER(_I)], "hybrid")
     ti_gemv_stream_part = (_I, [_I, _I, _I, _I, _I, ctypes.POINTER(_I)], "hybrid")
     ti_gemv_params_size = (_I, [], "hybrid")
     ti_chain_params_size = (_I, [], "hybrid")
