@@ -944,7 +944,7 @@ TI_DEVICE void gemv_body(const ChainParams& c, int cta, int ncta, uint8_t* smem)
       if (WT == W_INT8) {
 #pragma unroll
         for (int b = 0; b < 4; ++b)
-          acc[b] = ((float)(ah[0][b] + ah[1][b]) * 256.f + (p.K > kMaxIntK ? (float)((long long)al[0][b] + al[1][b]) : (float)(al[0][b] + al[1][b]))) * (b < 2 ? inv0 : inv1);
+          acc[b] = ((float)(ah[0][b] + ah[1][b]) * 256.f + (p.K > kMaxIntK ? (float)al[0][b] + (float)al[1][b] : (float)(al[0][b] + al[1][b]))) * (b < 2 ? inv0 : inv1);
       }
       if (p.T > 1) {
         // partial sums of the team meet in shared memory (two alternating slots: the barrier of exchange n+1
