@@ -347,18 +347,24 @@ static PairPlan pair_plan(int M, int n_tiles, int KS, int NT, bool may_cut) {
 static bool pair_may_cut(const void* part, size_t part_bytes, const void* tile_count, int n_count) {
   return part != nullptr && tile_count != nullptr && part_bytes >= (size_t)kPairs * 256 * 256 * 4 && n_count >= kPairs;
 }
-// Tokens of a pair's tile.  Batched decode: as few as hold the batch.  A few hundred tokens of few weight tiles: 64, where that
-// gives more pairs work in the one round there is (and the round would not be cut along k instead): a tile of 64 takes about 0.7 of one
-// of 128.  us with tiles of 128 / 64, int8: 5120 x 6144 at 65 / 128 / 192 tokens 19.4 / 15.4, 21.4 / 16.3, 21.9 / 16.7, 2048 x 6144 at 128 / 512
-// 20.8 / 14.6, 21.3 / 16.9, 6176 x 2048 at 128 12.2 / 9.7; bf16: 5120 x 6144 at 128 24.7 / 22.8, 2048 x 6144 at 512 33.3 / 23.3.  bf16 products of many tokens: 128-token tiles cost 0.62 of
-// 256-token ones (34816 x 5120 at 4096 tokens: 1143 us against 917), but leave fewer pairs idle in the last round (5120 x 6144 at
-// 4096 tokens: 221 against 257).
+// Tokens of a pair's tile.
+//   * Batched decode: as few as hold the batch.
+//   * bf16 products of many tokens: tiles of 128 tokens cost 0.62 of those of 256 (34816 x 5120 at 4096 tokens: 1143 us against 917), but
+//     may leave fewer pairs idle in the last round.
+//   * A few hundred tokens of few weight tiles: 64, where that gives more pairs work in the one round there is: a tile of 64 takes about 0.7
+//     of one of 128.  us with the larger tiles / 64, int8: 5120 x 6144 at 65 / 128 / 192 tokens 19.4 / 15.4, 21.4 / 16.3, 21.9 / 16.7, 2048 x 6144 at
+//     128 / 512 20.8 / 14.6, 21.3 / 16.9, 6176 x 2048 at 128 12.2 / 9.7; bf16: 5120 x 6144 at 128 24.7 / 22.8, 2048 x 6144 at 512 33.3 / 23.3.  Not where tiles
+//     of 128 would be cut along k instead, nor long products where those of 256 would: their partial results cost about 103 stages, a
+//     stage of a tile of 64 0.8 of theirs, since the weights' arrival bounds both (bf16, 256 cut / 64: 5120 x 17408 at 129 / 192 tokens 49.2 / 53.4,
+//     53.8 / 55.3, 5120 x 14336 43.7 / 45.1, 48.0 / 46.3, 5120 x 10240 36.5 / 34.1, 40.7 / 34.7, 2048 x 8192 at 129 / 256 30.0 / 19.9, 43.5 / 22.7).
 static int pair_tokens(bool bf16, int M, int n_tiles, int KS, bool may_cut) {
   if (M <= 64) return M <= 32 ? 32 : 64;
+  const PairPlan q128 = pair_plan(M, n_tiles, KS, 128, may_cut), q256 = pair_plan(M, n_tiles, KS, 256, may_cut);
+  const bool wide = bf16 && M > 128 && 0.62f * q128.rounds >= q256.rounds;
   const int tn = (n_tiles * 8 + 255) / 256, t64 = tn * ((M + 63) / 64);
-  if (t64 <= kPairs && t64 > tn * ((M + 127) / 128) && pair_plan(M, n_tiles, KS, 128, may_cut).slices == 1) return 64;
-  if (!bf16 || M <= 128) return 128;
-  return 0.62f * pair_plan(M, n_tiles, KS, 128, may_cut).rounds < pair_plan(M, n_tiles, KS, 256, may_cut).rounds ? 128 : 256;
+  const bool cut = wide ? q256.slices > 1 && 0.8f * KS >= q256.kb_per_split + 103 : q128.slices > 1;
+  if (t64 <= kPairs && t64 > tn * ((M + 127) / 128) && !cut) return 64;
+  return wide ? 256 : 128;
 }
 // Products with tiles enough for every SM without a k split.
 static bool pair_many(int M, int n_tiles) { return (n_tiles * 8 + 255) / 256 * ((M + 127) / 128) >= 120; }

@@ -218,6 +218,10 @@ int ti_gemm_w8a16(const void* w, const void* wscale, int n_tiles, int N, int K, 
   return ti::launch_gemm<128, false>(p, grid, st);
 }
 
+// Tokens of a tile of the products that pairs of CTAs take (gemm_pair.cuh): K of M x N x K in stages of 128 bytes, may_cut: whether the
+// workspace allows a k split.
+int ti_gemm_pair_tokens(int bf16, int M, int n_tiles, int KS, int may_cut) { return ti::pair_tokens(bf16 != 0, M, n_tiles, KS, may_cut != 0); }
+
 // The same for bf16 weights tiled [n_tiles][K/32][8][32] (lm_head, unquantised mode) and bf16 activations x [M][K]
 // (contiguous rows): tcgen05.mma kind::f16, fp32 accumulation.  epi 3 stores fp32 (logits).
 int ti_gemm_bf16(const void* w, int n_tiles, int N, int K, const void* x, int M, const void* resid, void* out, int ldo,

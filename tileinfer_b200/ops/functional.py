@@ -259,6 +259,7 @@ _l.register("ti_wait_flag_probe", _I, [_P, ctypes.c_uint, ctypes.c_ulonglong, _P
 
 _l.register("ti_quant_rows", _I, [_P, _I, _P, _F, _I, _I, _P, _P, _P, _P])
 _l.register("ti_gemm_epilogue_size", _I, [])
+_l.register("ti_gemm_pair_tokens", _I, [_I, _I, _I, _I, _I])
 _l.register("ti_gemm_bf16", _I, [_P, _I, _I, _I, _P, _I, _P, _P, _I, _I, _P, _P, ctypes.c_size_t, _P, _I, _P, _P])
 _l.register("ti_gemm_w8a16", _I, [_P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _I, _I, _P, _P, ctypes.c_size_t, _P, _I, _P, _P])
 _l.register("ti_latent_attn_params_size", _I, [], "latent")
