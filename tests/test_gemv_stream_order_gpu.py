@@ -1,4 +1,6 @@
 """What orders the parts of a chain of products through one ring per CTA (gemv_stream.cuh)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -58,6 +60,20 @@ def test_ctas_without_work(quant):
     from tileinfer_b200.ops import functional as F
     F.L()
     _agree(F, [(64, 128, F.EPI_ROWPAR), (256, 64, F.EPI_SWIGLU), (64, 128, F.EPI_ROWPAR), (136, 64, F.EPI_STORE)], 1, quant, 40)
+
+
+@pytest.mark.parametrize("quant", [True, False])
+def test_split_products_in_a_row(quant):
+    """Four products whose left-over tiles are cut along k: each uses the partial sums and counters of the one before again, with nothing
+    but the packets in between, and the third overwrites the first one's residual."""
+    from tileinfer_b200.ops import functional as F
+    F.L()
+    shapes = [(5120, 8192, F.EPI_ROWPAR), (16384, 5120, F.EPI_SWIGLU), (5120, 8192, F.EPI_ROWPAR), (8192, 5120, F.EPI_STORE)]
+    out = (ctypes.c_int * 7)()
+    for n, k, _ in shapes:
+        F.L().ti_gemv_stream_part(n // 8, k // (64 if quant else 32), 0, 0, F.NUM_SMS, out)
+        assert out[6] > 1
+    _agree(F, shapes, 1, quant, 12)
 
 
 def test_a_long_kernel_before_the_launch():

@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
             __threadfence();
           }
           finish = __shfl_sync(0xffffffffu, last, 0) != 0;
+          __syncwarp();                                      // the other lanes read behind lane 0's fence (a shuffle orders no memory)
           if (finish)
 #pragma unroll
             for (int m = 0; m < ROWS; ++m) {
