@@ -79,3 +79,13 @@ def test_rank_protocols_under_arrival_jitter():
                        capture_output=True, text=True, env=_env(), timeout=900, cwd=ROOT)
     assert r.returncode == 0, (r.stdout[-2500:], r.stderr[-1500:])
     assert " passed" in r.stdout and "failed" not in r.stdout
+
+
+def test_chains_of_products_under_arrival_jitter():
+    """One ring per CTA: chains whose rows go on as packets, or behind grid barriers, with random delays before every packet is sent or
+    waited for, every split counter, every barrier and the reading of the launch's tag."""
+    r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(ROOT, "tests", "test_gemv_stream_gpu.py"),
+                        os.path.join(ROOT, "tests", "test_gemv_stream_order_gpu.py"), "-q", "-x", "-k", "chain or without_work or in_a_row or barrier or long_kernel"],
+                       capture_output=True, text=True, env=_env(), timeout=900, cwd=ROOT)
+    assert r.returncode == 0, (r.stdout[-2500:], r.stderr[-1500:])
+    assert " passed" in r.stdout and "failed" not in r.stdout

@@ -204,6 +204,7 @@ template <int WT> TI_DEVICE void stage_row(const GemvParams& p, const RowChunks&
     if (packets == nullptr && c < chunks) x[j] = ld_x16(p.x + (size_t)c * 8);
   }
   if (packets != nullptr) {
+    jitter();
     PollLimit limit;
     bool missing = true;
     while (missing) {
@@ -211,7 +212,7 @@ template <int WT> TI_DEVICE void stage_row(const GemvParams& p, const RowChunks&
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
         const int c = tid + j * kThreads;
-        if (c >= chunks) continue;
+        if (c >= chunks || !TI_CHECK(c * 4 + 3, kStreamPacketBytes / 8, p.status)) continue;
         const uint4 a = packet_load2(packets + (size_t)c * 4), b = packet_load2(packets + (size_t)c * 4 + 2);
         missing = missing || a.y != tag || a.w != tag || b.y != tag || b.w != tag;
         x[j] = make_uint4(a.x, a.z, b.x, b.z);
@@ -406,7 +407,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
       if (op == 0) pdl_wait();
       else if (ROWS == 1 && flow.x[op]) Consumers::sync();   // all warps are done with the row before
       else sync_with_epilogue();                             // the epilogue warp has passed the grid barrier
-      if (ROWS == 1 && op == 0) tag = stream_tag(p0);
+      if (ROWS == 1 && op == 0) {
+        jitter();
+        tag = stream_tag(p0);
+      }
       if (dbg != nullptr && tid == 0) dbg[9 + 4 * op] = globaltimer_ns();
       const int lstride = limb_stride(p.K);
       if (ROWS == 1) stage_row<WT>(p, row, flow.x[op] ? stream_packets(p0, op - 1) : nullptr, tag, smem, lstride, scratch);
@@ -524,7 +528,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
         if (n >= p.N || !(x.two || row < 8)) return h;
         if (WT == W_INT8) h.scale = bf16_to_f(p.scale[n]);
         if (resid_from != nullptr) {
-          h.r[0] = packet_load(resid_from + (n >> 1));
+          if (TI_CHECK(n >> 1, kStreamPacketBytes / 8, p0.status)) h.r[0] = packet_load(resid_from + (n >> 1));
         } else if (p.epi == EPI_ROWPAR) {
 #pragma unroll
           for (int m = 0; m < ROWS; ++m)
@@ -553,7 +557,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
 #pragma unroll
           for (int w = 0; w < kWarps / 2; ++w) sum[m].add(reinterpret_cast<const typename Sum::T*>(e)[((half * (kWarps / 2) + w) * M + m) * 16 + row]);
           sum[m].add_other_half();
-          if (x.split && half == 0) __stcg(part_of + ((size_t)q.slice * M + m) * 16, sum[m].bits());
+          if (x.split && half == 0 && TI_CHECK((((long long)q.pair * q.slices + q.slice) * M + m) * 16 + row, kStreamPackets / 8, p0.status)) __stcg(part_of + ((size_t)q.slice * M + m) * 16, sum[m].bits());
         }
         __syncwarp();                                        // the slot has been read
         if (lane == 0) mbar_arrive(sum_free0 + 8 * slot);
@@ -562,6 +566,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
           ph ^= 1u;
         }
         if (x.split) {
+          jitter();
           __threadfence();
           __syncwarp();
           int last = 0;
@@ -605,7 +610,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
             const int sh = p.epi == EPI_SWIGLU ? 1 : 0;      // a result for each, or every other, weight row
             if (emit) {
               const float o2 = __shfl_xor_sync(0xffffffffu, o, 1 << sh);
-              if (live && half == 0 && (row & ((2 << sh) - 1)) == 0) packet_store(packets + (n >> (sh + 1)), pack_bf16(o, o2), tag);
+              jitter();
+              if (live && half == 0 && (row & ((2 << sh) - 1)) == 0 && TI_CHECK(n >> (sh + 1), kStreamPacketBytes / 8, p0.status)) packet_store(packets + (n >> (sh + 1)), pack_bf16(o, o2), tag);
             }
             if (live && half == 0 && (row & sh) == 0) static_cast<__nv_bfloat16*>(p.out)[(size_t)m * (p.epi == EPI_ROWPAR ? p.N : p.ldo) + (n >> sh)] = __float2bfloat16_rn(o);
           } else if (live && (v > am_v[m] || (v == am_v[m] && n < am_i[m]))) {
@@ -617,6 +623,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
       if (op + 1 < c.n_ops && !(ROWS == 1 && flow.x[op + 1])) {
         // ---- grid barrier: all results of this product are in L2
         if (dbg != nullptr && lane == 0) dbg[2 + op] = globaltimer_ns();
+        jitter();
         __threadfence();
         __syncwarp();
         if (lane == 0) {
