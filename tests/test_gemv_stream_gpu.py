@@ -1,6 +1,7 @@
-"""Products of up to 8 rows on one GPU, whose weights a CTA streams through one ring: sizes around a CTA's share of row tiles (none, a
-lone tile, left-over tiles cut along k, an odd number of those), k tiles around the 16 of a stage, rows up to 8, every epilogue, and
-chains whose rows go from product to product as packets, or behind a grid barrier.  Against fp64."""
+"""Products of one row on one GPU, whose weights a CTA streams through one ring: sizes around a CTA's share of row tiles (none, a
+lone tile, left-over tiles cut along k, an odd number of those), k tiles around the 16 of a stage, every epilogue, and chains whose rows
+go from product to product as packets, or behind a grid barrier; the same sizes with 2 and 8 rows, which take the other form except for
+bf16 rows too long to stage.  Against fp64."""
 import pytest
 import torch
 
