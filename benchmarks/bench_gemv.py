@@ -5,9 +5,11 @@ that every launch streams from HBM, not from the 126 MB L2.
     python benchmarks/bench_gemv.py [--timeline] [--chain]
 
 --chain times the four dependent products of a decoder layer (out_proj -> gate_up+SwiGLU -> down -> next
-in_proj, 27B shapes) in ONE launch, as the decode step runs them.
+in_proj, 27B shapes) in ONE launch, as the decode step runs them.  One row goes through one ring per CTA (gemv_stream.cuh), 2 to 16
+rows through a ring per warp (gemv_w8a16.cu); --teams concerns the latter.
 """
 import argparse
+import ctypes
 import os
 import sys
 
@@ -33,6 +35,8 @@ def _print_timeline(dbg, n_ops):
     t0 = t[:, 0].min()
 
     def row(nm, j):
+        if not bool(t[:, j].all()):            # a stamp that this form of the kernel does not write
+            return
         c = (t[:, j] - t0) / 1e3
         print(f"      {nm:22s} min {c.min():7.2f}  mean {c.mean():7.2f}  max {c.max():7.2f} us")
     row("start", 0)
@@ -46,6 +50,14 @@ def _print_timeline(dbg, n_ops):
         for k, nm in enumerate(("unit popped", "first chunk arrived", "tiles done")):
             row(f"op{op} warp0 last unit: {nm}", 24 + 4 * op + k)
     row("end", 5)
+
+
+def _geometry(ps, wt):
+    out = (ctypes.c_int * 3)()
+    F.L().ti_gemv_stream_plan(ctypes.byref(F.make_chain(ps)), wt, F.NUM_SMS, out)
+    if out[0]:
+        return f"one ring of {out[0]} x 16 KB per CTA"
+    return f"R={[p.R for p in ps]} T={[p.T for p in ps]}, {ps[0].stages} stages of {ps[0].tps} tiles per warp"
 
 
 def bench_chain(args):
@@ -89,7 +101,7 @@ def bench_chain(args):
     torch.cuda.synchronize()
     us = e0.elapsed_time(e1) * 1e3 / args.iters
     nbytes = sum(W.nbytes() for W in sets[0])
-    print(f"chain of 4 (27B layer, 1/{tp} shard) M={M} stages={chains[0][0].stages} T={[p.T for p in chains[0]]}: {us:7.2f} us  {nbytes / us / 1e3:7.1f} GB/s "
+    print(f"chain of 4 (27B layer, 1/{tp} shard) M={M}, {_geometry(chains[0], F.W_INT8)}: {us:7.2f} us  {nbytes / us / 1e3:7.1f} GB/s "
           f"({nbytes / 1e6:.0f} MB)")
     if args.timeline:
         _print_timeline(dbg, 4)
@@ -137,8 +149,7 @@ def main():
         e1.record()
         torch.cuda.synchronize()
         us = e0.elapsed_time(e1) * 1e3 / args.iters
-        p0 = ps[0]
-        print(f"{name:10s} N={N:6d} K={K:6d} M={M} R={p0.R} tps={p0.tps} stages={p0.stages} "
+        print(f"{name:10s} N={N:6d} K={K:6d} M={M} {_geometry(ps[:1], F.W_INT8)} "
               f"{us:7.2f} us  {N * K / us / 1e3:7.1f} GB/s")
         if args.timeline:
             _print_timeline(dbg, 1)
