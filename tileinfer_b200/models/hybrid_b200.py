@@ -114,10 +114,9 @@ class _ModelBase:
         # steps in which some sequence has at least this many tokens use the chunk-parallel DeltaNet kernels
         self.gdn_chunk_min_tokens = int(os.environ.get("TI_GDN_CHUNK_MIN", "32"))
         self.gdn_ws = F.GdnChunkWorkspace(dev)
-        # more rows than this: tcgen05 GEMM; the persistent GEMV chain serves single rows.  (Measured on the 27B model,
-        # one GPU, ms per decode step: 1 row 6.6 on the GEMV chain; 2 / 3 / 4 rows 8.2 / - / 10.5 on the GEMV against
-        # 6.9 / 7.4 / 7.4 on the GEMM; 8 rows 16.0 on the GEMV, whose long-k products then need two passes over the
-        # weights, 7.7 on the GEMM.)
+        # more rows than this: tcgen05 GEMM; the persistent GEMV chain serves single rows.  (The four products of a 27B layer, one GPU,
+        # us: 1 row 69 on the GEMV chain; 2 / 4 rows 110 / 141 on the GEMV chain against 87 / 87 with quantisations on the GEMM; the model's
+        # decode step 5.2 ms at 1 row on the GEMV chain, 6.7 at 2 on the GEMM.)
         self.gemm_min_rows = int(os.environ.get("TI_GEMM_MIN_ROWS", "1"))
 
     # ------------------------------------------------------------------ weights: build / on-disk shard cache

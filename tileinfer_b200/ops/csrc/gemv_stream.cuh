@@ -15,7 +15,8 @@
 //     and 4 MMAs per KB in int8 (one row: 3 and 2), where lanes without an activation row load nothing;
 //   * sums of a unit (two row tiles) of the 16 warps meet in shared memory, as integers for int8 weights (so they are exact
 //     whatever the split); one warp adds them up and runs the epilogue, its operands requested ahead;
-//   * one row goes to the next product as packets that its consumers poll, several behind a grid barrier.
+//   * one row goes to the next product as packets that its consumers poll; several rows, and one that registers do not hold, behind a
+//     grid barrier.
 // Roles (608 threads): warps 0..15 consume, warps 16 and 18 copy, warp 17 is the epilogue.  Every wait is bounded.
 #pragma once
 
@@ -713,7 +714,11 @@ static bool stream_plan(const ChainParams& c, int wt, int ncta, StreamPlan& q) {
 }
 
 // Which products of a launch hand their row on as packets.  Only where a row is exactly the results of the product before; and
-// nowhere if a product reads or overwrites what another one of the launch writes in any other way, which needs the barrier's order.
+// nowhere if a product reads or overwrites what an earlier one of the launch writes in any other way, which needs the barrier's order.
+// What an earlier product READS from memory may be overwritten without a barrier (hidden rows go back and forth between two buffers: the
+// third product of a layer's chain writes the first one's residual): no CTA has a result of product j before it holds the whole row of
+// product j - 1, and so on back to i, and a result of product i is sent only after all that it is made of has been read; what a CTA
+// without a part in product i reads later goes into no result.
 static StreamFlow stream_flow(const ChainParams& c, int rows) {
   StreamFlow f = {};
   auto width = [&](int i) { return c.op[i].epi == EPI_SWIGLU ? c.op[i].N / 2 : c.op[i].N; };

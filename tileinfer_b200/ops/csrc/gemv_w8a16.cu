@@ -41,8 +41,8 @@ struct GemvParams {
   const __nv_bfloat16* norm_w;   // XNORM: RMSNorm weight (1+w convention) [K]
   void* out;                     // see epilogues
   const __nv_bfloat16* resid;    // ROWPAR: residual in [M, N]
-  float* ws;                     // split-k partials [units][128]
-  unsigned* counters;            // [n_tiles], zero between launches
+  float* ws;                     // gemv_stream.cuh: sums of the slices of cut tiles, from kStreamPackets bytes on packets; or null (neither)
+  unsigned* counters;            // gemv_stream.cuh: slices done of a pair of cut tiles, zero between launches
   const unsigned* step_ptr;      // device step counter (tag source), ROWPAR with tp > 1
   unsigned* status;              // error bits
   uint64_t peer_ll[kMaxRanks];   // packet buffers of all ranks as mapped in this process
@@ -55,8 +55,9 @@ struct GemvParams {
   int T;                         // team size (1..16 adjacent warps of a CTA share a unit, each a k-slice)
   unsigned long long* dbg;       // optional [ncta][32] globaltimer stamps of warp 0 (profiling aid): 0 start, 1 ring
                                  // primed, 2..4 all warps of the CTA reached the barrier before product 1..3, 5 end; per product op at 8 + 4*op:
-                                 // marker reached, barrier passed, x staged, last unit done
-  int* sched;                    // dynamic scheduling state: [0] launches finished, [1] CTAs finished, [8 + 3*16] tickets
+                                 // marker reached, barrier passed, x staged, last unit done; a form leaves out what it has no place for
+  int* sched;                    // [1] CTAs finished, [2] grid barriers, both zero between launches; [3] launches of gemv_stream.cuh, the tag
+                                 // of their packets; [8 + 16 * product] tickets of this file's form, zero between launches
   int tps;                       // 512-byte tiles per ring stage (4, 8 or 16)
   int xmode, epi;                // XGLOBAL | XNORM ; EPI_*
   int R;                         // row tiles (of 8 weight rows) per unit: 1 or 2
@@ -67,8 +68,8 @@ struct GemvParams {
 };
 
 // Up to four dependent products run back to back in one launch (e.g. out_proj -> gate_up -> down -> the
-// next layer's in_proj): a grid barrier separates them, the weight streams of the warps run ahead into the
-// next product while the barrier and the activation staging take place, so HBM never drains between them.
+// next layer's in_proj): a grid barrier separates them, or the row goes on as packets (gemv_stream.cuh, and between two ranks); the
+// weight streams run ahead into the next product while the barrier and the activation staging take place.
 constexpr int kMaxChain = 4;
 struct ChainParams {
   int n_ops;

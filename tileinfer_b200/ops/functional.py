@@ -447,7 +447,9 @@ def status_ptr() -> int:
 
 
 class GemvWorkspace:
-    """Split-k partial buffer and per-tile arrival counters shared by all GEMV launches of a stream."""
+    """What the GEMV launches of a stream share: sums of cut tiles and packets (`ws`; 1 MB of it is used), counters of cut tiles, and the
+    scheduling state with the launch counter (GemvParams.sched).  With less than 1 MB or 148 counters nothing is cut and rows go from
+    product to product behind grid barriers."""
 
     def __init__(self, device="cuda", max_units: int = 1 << 16, max_tiles: int = 1 << 16):
         self.ws = torch.zeros(max_units * 128, dtype=torch.float32, device=device)      # (zero: a tag no packet has)
@@ -489,8 +491,6 @@ def make_gemv_params(W: LinearW, x, out, M, *, xmode=XGLOBAL, epi=EPI_STORE, nor
     p._xb = x_smem_bytes(W.wt, xmode, M, W.K, W.K)
     p.xmode, p.epi = xmode, epi
     p.xll = int(bool(xll))
-    if ws is None:
-        ws = default_workspace()
     p.sched = ptr(ws.sched)
     p.status = status or status_ptr()
     p.tp, p.rank, p.order, p.m_cap = 1, 0, order, 0
